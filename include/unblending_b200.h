@@ -50,19 +50,21 @@ typedef struct unblending_solver_options {
                                    Pixels the learned start leaves unsolved get the plain solve from the
                                    reference's start (FP64 precision: the FP64 solve; FP32 precision with
                                    resolve_misses: the FP32 solve, and what that misses the FP64 re-solve). */
-    int32_t fp64_variant;       /* FP64 solve and re-solve: -1 default; history in shared memory with 0
-                                   uncapped registers, 1 capped for 2 blocks per SM; 2 history in global memory,
+    int32_t fp64_variant;       /* FP64 solve and re-solve: -1 default, one pixel per lane (first passes of up to
+                                   three layers and fewer than 32,768 pixels, and calls that set
+                                   threads_per_block, run the quad kernels 3 and 7). Quad kernels (four or three
+                                   lanes per pixel), history in shared memory with 0 uncapped registers, 1 capped for 2 blocks per SM; 2 history in global memory,
                                    x/g/d in shared memory, evaluation rolled, 3 blocks per SM; 3 as 2 with the
                                    start and bounds in global memory, 4 blocks per SM; 4/5 as 3/2 with three
                                    lanes per pixel where the alphas are pinned (refinement); 6 as 3 (first pass)
                                    and 5 (refinement) with the bookkeeping rolled over the layers; 7 the
                                    refinement of 6 with its start and bounds in global memory, 4 blocks per SM
-                                   (first passes run 3). Default: 3 for the first pass, 7 for the refinement.
-                                   Every variant gives the same results. */
+                                   (first passes run 3). Every variant, and the default, gives the same
+                                   results. */
     int32_t fp32_outer;         /* FP32 precision with resolve_misses: outer steps of the FP32 solve before a
                                    pixel is left to the FP64 re-solve (default 9; 0 = outer);
                                    a pixel stopped there unconverged is always re-solved */
-    int32_t gradient_quorum;    /* scheduling of the pixels of one warp: an evaluation with a gradient runs when
+    int32_t gradient_quorum;    /* quad kernels: scheduling of the pixels of one warp: an evaluation with a gradient runs when
                                    at least gradient_quorum/8 of the warp's pixels need one (or none needs a
                                    value alone); the others wait one evaluation. 0 = never wait. Results do not
                                    depend on it. Default 4 (FP64 solves of the 1024x1024 five-layer image:
@@ -76,7 +78,7 @@ typedef struct unblending_solver_options {
                                    together take similar paths through the method; 0 image order. Results do not
                                    depend on it. A caller built against the previous layout, whose struct_size
                                    ends before this field, gets the default. */
-    int32_t defer_outer;        /* FP64 refinement solve (kernel variant 7, the default): a pixel still unsolved
+    int32_t defer_outer;        /* FP64 refinement solve on quads (kernel variant 7): a pixel still unsolved
                                    when it reaches this outer step leaves the solve launch with its state and is
                                    resumed, with the other such pixels, by a second launch right behind it; the
                                    pixels the method struggles with then share warps. 0 = no deferral. Results do

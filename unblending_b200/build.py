@@ -30,6 +30,7 @@ COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-I" + os.pat
 # reference's CUDA build.
 UNITS = [
     *[(f"solver_l{L}.cu", ["--fmad=false"]) for L in range(1, 9)],
+    *[(f"lane_l{L}.cu", ["--fmad=false"]) for L in range(1, 9)],
     ("solver_launch.cu", []),
     ("filter.cu", ["--fmad=false"]),
     ("noalloc.cu", []),

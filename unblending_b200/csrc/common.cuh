@@ -19,6 +19,7 @@ template <class T> struct Models {
     T prec[kMaxLayers][9];
     int mode[kMaxLayers];
     int X[kMaxLayers], Y[kMaxLayers], Z[kMaxLayers];
+    T fX[kMaxLayers], fY[kMaxLayers], fZ[kMaxLayers];   // X, Y, Z in the arithmetic type
     // Branch-free form of the ten piecewise-bilinear modes:
     //   B = c0 + cs s + cd d + csd s d, coefficient set [0] where
     //   t = ka s + kb d + kc satisfies t < 0 (strict) or t <= 0, else set [1];
@@ -66,6 +67,28 @@ struct SolverControls {
     int cap_is_miss = 0;               // a pixel that reaches the outer cap unconverged is a miss
     int frozen_stop = 0;               // stop after this many outer steps that move neither x nor the best point
 };
+
+// Lane kernels (lane_solver.cuh), one pixel per lane: blocks of four warps.
+// A lane's global-memory records (32 bytes: one layer's three colours and
+// alpha) are the steps and gradient changes of the L-BFGS ring, which has a
+// spare slot that an accepted step fills before its curvature test, the best
+// point, and the outer step's start.
+constexpr int kLaneBlock = 128;
+constexpr int kLaneRing = kHistory + 1;
+__host__ __device__ constexpr int lane_records(int L) { return (2 * kLaneRing + 2) * L; }
+// Shared memory of a lane in 16-byte units: x, g, d (4 L values each; d's area
+// also takes the two-loop recursion's coefficients, six pairs).
+__host__ __device__ constexpr int lane_smem_units(int L) { return 4 * L + (2 * L > kHistory ? 2 * L : kHistory); }
+__host__ __device__ constexpr int lane_smem_bytes(int L) { return lane_smem_units(L) * kLaneBlock * 16; }
+// Resident blocks per SM: what shared memory holds for many layers (61 KB a
+// block at five layers, 98 KB at eight), and enough registers for the
+// direction's unrolled loops for few (a third block more at five layers, 128
+// registers instead of 168, spilled 600 bytes and was slower).
+__host__ __device__ constexpr int lane_blocks_per_sm(int L) { return L <= 4 ? 4 : L <= 6 ? 3 : 2; }
+__host__ __device__ constexpr int lane_blocks(int L, int sms) { return lane_blocks_per_sm(L) * sms; }
+__host__ __device__ constexpr size_t lane_history_bytes(int L, int sms) {
+    return size_t(lane_blocks(L, sms)) * kLaneBlock * 32 * size_t(lane_records(L));
+}
 
 // Words a lane of a deferred pixel keeps (SolveArgs::defer_state): x, the
 // best point and the start seed (L each), up to L multipliers, and seven

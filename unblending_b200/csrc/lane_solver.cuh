@@ -1,0 +1,1002 @@
+// Per-pixel augmented-Lagrangian / projected L-BFGS solve, one pixel per lane
+// (FP64).
+//
+// The method, its FP64 arithmetic and its operation order are those of
+// solver.cuh (rounded multiplies and adds; a pixel's sums over the three
+// channels and the alphas are added in the tree in which a quad's lanes add
+// theirs), so outputs, statuses and counters equal its kernels' bit for bit.
+//
+// Why one pixel per lane: on a quad, all four lanes repeat the composite alpha
+// chain and the 3x3 colour prior, lane 3 idles through the colour arithmetic,
+// every sum costs shuffles, and a trip issues about four times the
+// instructions a pixel needs. Here a pixel's three channels are three
+// independent chains of one lane. The price is state: x, g and d (12 L
+// doubles) live in shared memory (conflict-free 16-byte accesses), the L-BFGS
+// ring, the best point and the outer step's start in global memory, one
+// 32-byte sector per layer and lane, so a lane's loads use whole sectors
+// whatever ring slot its neighbours are at.
+//
+// Phases: a block's lanes are at different actions (a line-search trial, a
+// gradient, a new direction, the end of an outer step). The block runs the
+// actions as phases, all warps at once: every trip evaluates the lanes with a
+// trial, and the other actions run when a share of the block's lanes waits
+// for them (or none has a trial). With each warp on its own schedule, the
+// instruction cache thrashed between the phases' code (85 KB; 4 to 7 cycles
+// of fetch stall per issue, 75 + 45 ms for the two passes of the 1024x1024
+// five-layer image); with the block in phase the stall is 0.14 cycles (51 + 29
+// ms, against 134 + 99 on quads).
+//
+// An accepted trial needs its gradient once; the lane's values repeat their
+// evaluation during the next trial phase, beside the lanes that evaluate
+// anyway, and keep what the reverse sweep reads.
+#pragma once
+#include "blend.cuh"
+#include "common.cuh"
+#include "quotient.hpp"
+#include "solver.cuh"
+
+namespace unb {
+
+__device__ __forceinline__ double mul_add(double a, double b, double c) { return __dadd_rn(__dmul_rn(a, b), c); }
+
+// Blend values of three channels of one layer (blend_value of each).
+__device__ __forceinline__ void blend_value3(int mode, const double* s, const double* d, double* f) {
+    const double eps = 1e-5;
+    switch (mode) {
+    case 0:
+#pragma unroll
+        for (int c = 0; c < 3; ++c) f[c] = s[c];
+        return;
+    case 1:
+#pragma unroll
+        for (int c = 0; c < 3; ++c) f[c] = s[c] * d[c];
+        return;
+    case 2:
+#pragma unroll
+        for (int c = 0; c < 3; ++c) f[c] = 1.0 - (1.0 - s[c]) * (1.0 - d[c]);
+        return;
+    case 3:
+    case 8:
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double t = mode == 3 ? d[c] : s[c];
+            const double lowv = 2.0 * s[c] * d[c], highv = 1.0 - 2.0 * (1.0 - s[c]) * (1.0 - d[c]);
+            f[c] = t <= 0.5 ? lowv : highv;
+        }
+        return;
+    case 4:
+#pragma unroll
+        for (int c = 0; c < 3; ++c) f[c] = s[c] < d[c] ? s[c] : d[c];
+        return;
+    case 5:
+#pragma unroll
+        for (int c = 0; c < 3; ++c) f[c] = s[c] < d[c] ? d[c] : s[c];
+        return;
+    case 6:     // d / (1 - s), and Burn, 1 - (1 - d) / s, by the same code
+    case 7:
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double p = mode == 6 ? d[c] : 1.0 - d[c], q = mode == 6 ? 1.0 - s[c] : s[c];
+            const double v = quotient(p, q, __drcp_rn(q));
+            const double r = p < eps ? 0.0 : (q < eps ? 1.0 : (v < 1.0 ? v : 1.0));
+            f[c] = mode == 6 ? r : 1.0 - r;
+        }
+        return;
+    case 9:
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double lowv = d[c] - (1.0 - 2.0 * s[c]) * d[c] * (1.0 - d[c]);
+            const double highv = d[c] + (2.0 * s[c] - 1.0) * (softlight_g(d[c]) - d[c]);
+            f[c] = s[c] <= 0.5 ? lowv : highv;
+        }
+        return;
+    case 10:
+#pragma unroll
+        for (int c = 0; c < 3; ++c) f[c] = s[c] < d[c] ? d[c] - s[c] : s[c] - d[c];
+        return;
+    case 11:
+#pragma unroll
+        for (int c = 0; c < 3; ++c) f[c] = s[c] + d[c] - 2.0 * s[c] * d[c];
+        return;
+    case 12:
+#pragma unroll
+        for (int c = 0; c < 3; ++c) f[c] = s[c] + d[c];
+        return;
+    default:
+#pragma unroll
+        for (int c = 0; c < 3; ++c) f[c] = 0.0;
+        return;
+    }
+}
+
+// Blend values and partials of three channels (blend_all of each).
+__device__ __forceinline__ void blend_all3(int mode, const double* s, const double* d, double* f, double* fs,
+                                           double* fd) {
+    const double eps = 1e-5;
+    if (mode == 6 || mode == 7) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double p = mode == 6 ? d[c] : 1.0 - d[c], q = mode == 6 ? 1.0 - s[c] : s[c];
+            const double y = __drcp_rn(q), qq = q * q;
+            const double v = quotient(p, q, y), g = quotient(p, qq, __drcp_rn(qq));
+            const bool dark = p < eps, flat = dark || q < eps || 1.0 < v;
+            const double r = dark ? 0.0 : (flat ? 1.0 : v);
+            f[c] = mode == 6 ? r : 1.0 - r;
+            fs[c] = flat ? 0.0 : g;
+            fd[c] = flat ? 0.0 : y;
+        }
+    } else {
+        // The remaining modes have no division but SoftLight's, which keeps
+        // the one-channel form.
+        switch (mode) {
+        case 0:
+#pragma unroll
+            for (int c = 0; c < 3; ++c) { f[c] = s[c]; fs[c] = 1.0; fd[c] = 0.0; }
+            return;
+        case 1:
+#pragma unroll
+            for (int c = 0; c < 3; ++c) { f[c] = s[c] * d[c]; fs[c] = d[c]; fd[c] = s[c]; }
+            return;
+        case 2:
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double p = 1.0 - s[c], q = 1.0 - d[c];
+                f[c] = 1.0 - p * q; fs[c] = q; fd[c] = p;
+            }
+            return;
+        case 3:
+        case 8:
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double t = mode == 3 ? d[c] : s[c];
+                const bool low = t <= 0.5;
+                const double a = low ? s[c] : 1.0 - s[c], b = low ? d[c] : 1.0 - d[c];
+                const double p = 2.0 * a * b;
+                f[c] = low ? p : 1.0 - p; fs[c] = 2.0 * b; fd[c] = 2.0 * a;
+            }
+            return;
+        case 4:
+        case 5:
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const bool less = s[c] < d[c], src = mode == 4 ? less : !less;
+                f[c] = src ? s[c] : d[c]; fs[c] = src ? 1.0 : 0.0; fd[c] = src ? 0.0 : 1.0;
+            }
+            return;
+        case 10:
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const bool less = s[c] < d[c];
+                f[c] = less ? d[c] - s[c] : s[c] - d[c]; fs[c] = less ? -1.0 : 1.0; fd[c] = less ? 1.0 : -1.0;
+            }
+            return;
+        case 11:
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                f[c] = s[c] + d[c] - 2.0 * s[c] * d[c]; fs[c] = 1.0 - 2.0 * d[c]; fd[c] = 1.0 - 2.0 * s[c];
+            }
+            return;
+        case 12:
+#pragma unroll
+            for (int c = 0; c < 3; ++c) { f[c] = s[c] + d[c]; fs[c] = 1.0; fd[c] = 1.0; }
+            return;
+        case 9:
+#pragma unroll
+            for (int c = 0; c < 3; ++c) blend_all<double>(9, s[c], d[c], f[c], fs[c], fd[c]);
+            return;
+        default:
+#pragma unroll
+            for (int c = 0; c < 3; ++c) { f[c] = 0.0; fs[c] = 0.0; fd[c] = 0.0; }
+            return;
+        }
+    }
+}
+
+// ----------------------------------------------------------------- storage --
+// A lane's four values of one layer (three colours, alpha) as one 32-byte
+// sector of global memory.
+__device__ __forceinline__ void load_rec(const double* p, double* v) {
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void store_rec(double* p, double a, double b, double c, double d) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+
+extern __shared__ __align__(16) unsigned char lane_smem[];
+
+// Eighths of a block's live lanes that start a phase: the end of an outer
+// step, a direction, a gradient. Measured on the 1024x1024 five-layer image,
+// first pass + refinement in ms: 4, 2, 2: 50.8 + 29.2; 2, 2, 2: 52.6 + 29.8; 4, 3,
+// 2: 52.5 + 32.6; 4, 2, 3: 49.6 + 30.4; 3, 1, 2: 53.9 + 29.6.
+constexpr int kOuterQuorum = 4, kDirectionQuorum = 2, kGradientQuorum = 2;
+enum : int { kLaneIdle = 0, kLaneTrial, kLaneOuter, kLaneGrad, kLaneDir, kLaneSteep, kLaneEnd, kLaneFetch };
+
+template <int L, bool REFINE, bool BATCH> struct LaneSolver {
+    static constexpr int NV = REFINE ? 3 : 4;    // components of a layer that the method moves
+    const Models<double>* models_;
+    const SolverControls& ctl;
+    const SolveArgs& a;
+    const int lane = threadIdx.x & 31;
+    double* rec_base;
+    size_t rec_stride;      // doubles between a lane's records
+    int job_id = -1;
+    uint32_t n_value = 0, n_grad = 0;
+
+    // Pixel.
+    int state = kLaneFetch, pixel = 0, gidx = 0;
+    double target[3];
+    double lam[NV], resx[NV];
+    double rho, f, oldnorm, step, best_norm, best_energy, ss_kept;
+    int start, outer, it, bt, valid, next, frozen;
+    bool second;        // the line search's steepest-descent attempt
+    bool from_trial;    // kLaneGrad: the point is an accepted trial (else the outer step's start)
+    bool small_change, best_moved, have_best;
+    bool pending = false;   // this trip computes the gradient
+
+    __device__ LaneSolver(const Models<double>* m, const SolverControls& c, const SolveArgs& args)
+        : models_(m), ctl(c), a(args) {
+        rec_stride = size_t(gridDim.x) * kLaneBlock * 4;
+        rec_base = static_cast<double*>(a.history) + (size_t(blockIdx.x) * kLaneBlock + threadIdx.x) * 4;
+        if constexpr (BATCH) models_ = static_cast<const Models<double>*>(a.models);
+    }
+
+    // ------------------------------------------------------------ storage --
+    __device__ __forceinline__ double2* slot(int unit) const {
+        return reinterpret_cast<double2*>(lane_smem) + unit * kLaneBlock + threadIdx.x;
+    }
+    __device__ __forceinline__ void get(int vec, int l, double* v) const {
+        const double2* p = slot(vec * 2 * L + 2 * l);
+        const double2 u = p[0], w = p[kLaneBlock];
+        v[0] = u.x; v[1] = u.y; v[2] = w.x; v[3] = w.y;
+    }
+    __device__ __forceinline__ void put(int vec, int l, double v0, double v1, double v2, double v3) const {
+        double2* p = slot(vec * 2 * L + 2 * l);
+        p[0] = make_double2(v0, v1);
+        p[kLaneBlock] = make_double2(v2, v3);
+    }
+    enum : int { kX = 0, kG = 1, kD = 2 };
+    __device__ __forceinline__ double* rec(int k) const { return rec_base + size_t(k) * rec_stride; }
+    __device__ __forceinline__ double* ring(int s, int w, int l) const { return rec((s * 2 + w) * L + l); }
+    __device__ __forceinline__ double* best_rec(int l) const { return rec(2 * kLaneRing * L + l); }
+    __device__ __forceinline__ double* ox_rec(int l) const { return rec((2 * kLaneRing + 1) * L + l); }
+
+    __device__ __forceinline__ void count(int k, uint32_t n = 1) const { if (a.counters) a.counters[5 * size_t(gidx) + k] += n; }
+    __device__ __forceinline__ const double* image() const {
+        if constexpr (BATCH) return a.jobs[job_id].image; else return a.image;
+    }
+    __device__ __forceinline__ size_t pixels() const {
+        if constexpr (BATCH) return size_t(a.jobs[job_id].n); else return size_t(a.n);
+    }
+    __device__ __forceinline__ bool fixed_bounds(int l, int c) const {
+        return l == 0 && (c == 3 ? a.opaque != 0 : (REFINE && a.smooth != 0));
+    }
+    __device__ __forceinline__ bool fixed_at(int l, int c, double x, double g) const {
+        return fixed_bounds(l, c) || (x <= 0.0 && g > 0.0) || (x >= 1.0 && g < 0.0);
+    }
+    __device__ __forceinline__ static double clamp01(double v) { return v < 0.0 ? 0.0 : (v > 1.0 ? 1.0 : v); }
+
+    // The per-channel partial sums, added as the lanes of a group add theirs.
+    __device__ __forceinline__ static double sum(const double* v) {
+        if constexpr (REFINE) return (v[0] + v[1]) + v[2];
+        else return (v[0] + v[1]) + (v[2] + v[3]);
+    }
+
+    // ------------------------------------------------------------ forward --
+    // One layer of the composite: A, pc in/out.
+    __device__ __forceinline__ void compose(const Models<double>& m, int l, const double* t, double av, double& A,
+                                            double* pc) const {
+        if (l == 0) {
+            A = av;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) pc[c] = t[c];
+            return;
+        }
+        const double dd = A, X = m.fX[l], Y = m.fY[l], Z = m.fZ[l];
+        const double n_dd = 1.0 - dd, n_av = 1.0 - av;
+        const double ya = __dmul_rn(Y * av, n_dd), zd = __dmul_rn(Z * dd, n_av);
+        const double Al = __dadd_rn(zd, mul_add(X * av, dd, ya));
+        double fv[3];
+        blend_value3(m.mode[l], t, pc, fv);
+        const double y = __drcp_rn(Al);
+        const bool big = Al > 1e-12;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double pre = mul_add(zd, pc[c], mul_add(fv[c] * av, dd, ya * t[c]));
+            const double q = quotient(pre, Al, y);
+            pc[c] = big ? q : pre;
+        }
+        A = Al;
+    }
+
+    // Trial point of layer l: x + step d within bounds (the fixed values have
+    // d = 0 and x in [0, 1]), or x itself at the start of an outer step.
+    __device__ __forceinline__ void trial(const double* x, const double* d, bool at_x, double* t) const {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (REFINE && c == 3) { t[c] = x[c]; continue; }
+            const double v = clamp01(mul_add(step, d[c], x[c]));
+            t[c] = at_x ? x[c] : v;
+        }
+    }
+
+    // Evaluates the objective at the trial point (kLaneTrial) or at x
+    // (kLaneOuter) and decides the trial. A lane whose point is accepted and
+    // whose gradient comes next (kLaneGrad) repeats its evaluation beside the
+    // others', at no cost of its own, and keeps what the reverse sweep needs:
+    // x becomes the accepted point, its step goes to the ring's free slot, and
+    // d's slots take the composite's colours and alpha.
+    __device__ __forceinline__ void forward() {
+        const Models<double>& m = *models_;
+        const bool keep = state == kLaneGrad, at_x = state == kLaneOuter || (keep && !from_trial);
+        bool moved = false;     // some component moved by at least the inner tolerance
+        const double tol_lo = ctl.inner_tolerance * (1.0 - 0x1p-48), tol_hi = ctl.inner_tolerance * (1.0 + 0x1p-48);
+        double sl[NV], mo[NV], A = 0.0, pc[3], energy = 0.0, asum = 0.0;
+#pragma unroll
+        for (int c = 0; c < NV; ++c) { sl[c] = 0.0; mo[c] = 0.0; }
+#pragma unroll 1
+        for (int l = 0; l < L; ++l) {
+            double x[4], d[4], g[4], t[4];
+            get(kX, l, x); get(kD, l, d); get(kG, l, g);
+            trial(x, d, at_x, t);
+#pragma unroll
+            for (int c = 0; c < NV; ++c) {
+                const double delta = t[c] - x[c];
+                sl[c] = mul_add(g[c], delta, sl[c]);
+                mo[c] = mul_add(delta, delta, mo[c]);
+            }
+            const double av = t[3];
+            const double d0 = t[0] - m.mean[l][0], d1 = t[1] - m.mean[l][1], d2 = t[2] - m.mean[l][2];
+            const double* P = m.prec[l];
+            const double v0 = mul_add(P[2], d2, mul_add(P[0], d0, P[1] * d1));
+            const double v1 = mul_add(P[5], d2, mul_add(P[3], d0, P[4] * d1));
+            const double v2 = mul_add(P[8], d2, mul_add(P[6], d0, P[7] * d1));
+            const double D = mul_add(d2, v2, mul_add(d0, v0, d1 * v1));
+            energy = mul_add(av, D, energy);
+            asum += av;
+            compose(m, l, t, av, A, pc);
+            if (keep) {
+                if (!at_x) {
+                    double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+                    for (int c = 0; c < NV; ++c) {
+                        s[c] = t[c] - x[c];
+                        // |s| / (1 + |x|) against the tolerance without the
+                        // division, except where rounding could decide.
+                        const double w = 1.0 + fabs(x[c]), as = fabs(s[c]);
+                        if (!(as < tol_lo * w)) moved = moved || as > tol_hi * w || step_reaches(as, w, ctl.inner_tolerance);
+                    }
+                    store_rec(ring(next, 0, l), s[0], s[1], s[2], s[3]);
+                    put(kX, l, t[0], t[1], t[2], t[3]);
+                }
+                put(kD, l, pc[0], pc[1], pc[2], A);
+            }
+        }
+        if (keep) {
+            small_change = small_change || !moved;
+            ss_kept = sum(mo);
+            return;
+        }
+        if (!REFINE) energy += 0.01 * asum;
+        double res[NV], terms[NV], nn[NV];
+#pragma unroll
+        for (int c = 0; c < NV; ++c) {
+            res[c] = c < 3 ? pc[c < 3 ? c : 0] - target[c < 3 ? c : 0] : A - 1.0;
+            terms[c] = mul_add(0.5 * rho * res[c], res[c], -(lam[c] * res[c]));
+            nn[c] = res[c] * res[c];
+        }
+        const double norm = sum(nn), value = energy + sum(terms);
+        const double slope = sum(sl), motion = sum(mo);
+
+        // A trial that does not move ends the attempt, unevaluated.
+        if (!at_x && motion == 0.0) { attempt_failed(); return; }
+        const double tol2 = ctl.outer_tolerance * ctl.outer_tolerance;
+        const bool feasible = norm < tol2;
+        if (isfinite(energy) && isfinite(norm) &&
+            (!have_best || (feasible && (best_norm >= tol2 || energy < best_energy)) ||
+             (!feasible && best_norm >= tol2 && norm < best_norm))) {
+            have_best = true; best_norm = norm; best_energy = energy; best_moved = true;
+#pragma unroll 1
+            for (int l = 0; l < L; ++l) {
+                double x[4], d[4], t[4];
+                get(kX, l, x); get(kD, l, d);
+                trial(x, d, at_x, t);
+                store_rec(best_rec(l), t[0], t[1], t[2], t[3]);
+            }
+        }
+        // Evaluations are counted as the method makes them: a first trial
+        // with its gradient, and a later trial that is accepted once more,
+        // with its gradient.
+        const bool counted_grad = at_x || (bt == 0 && ctl.gradient_on_first_trial);
+        count(0); ++n_value;
+        if (counted_grad) { count(1); ++n_grad; }
+        if (at_x) {
+            f = value;
+            oldnorm = norm;
+            valid = 0; next = 0; it = 0;
+            from_trial = false;
+            state = kLaneGrad;
+        } else {
+            count(3);
+            if (slope < 0.0 && isfinite(value) && value <= f + 1e-4 * slope) {
+                if (!counted_grad) { count(0); count(1); ++n_value; ++n_grad; }
+                const double delta = fabs(f - value), size = 0.5 * (fabs(f) + fabs(value));
+                small_change = delta < ctl.inner_tolerance * size;
+                f = value;
+                from_trial = true;
+                state = kLaneGrad;
+            } else {
+                step *= 0.5;
+                if (++bt >= 32) attempt_failed();
+                return;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < NV; ++c) resx[c] = res[c];
+    }
+
+    __device__ __noinline__ static bool step_reaches(double as, double w, double tol) { return !(as / w < tol); }
+
+    // The line search ran out of trials: once more from steepest descent,
+    // then the end of the inner solve.
+    __device__ __forceinline__ void attempt_failed() {
+        valid = 0; next = 0;
+        state = second ? kLaneEnd : kLaneSteep;
+    }
+
+    // ----------------------------------------------------------- backward --
+    // Gradient at the evaluated point (kLaneGrad, after forward()), and the
+    // accepted step's curvature pair and termination test.
+    __device__ __forceinline__ void backward() {
+        const Models<double>& m = *models_;
+        const bool at_x = !from_trial;
+        // Reverse sweep; layer l's slot of d turns from its composite into its gradient.
+        double adj[3], adj3 = REFINE ? 0.0 : rho * resx[NV - 1] - lam[NV - 1];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) adj[c] = rho * resx[c] - lam[c];
+#pragma unroll 1
+        for (int l = L - 1; l >= 0; --l) {
+            double t[4], ng[4];
+            get(kX, l, t);
+            const double av = t[3];
+            {
+                const double d0 = t[0] - m.mean[l][0], d1 = t[1] - m.mean[l][1], d2 = t[2] - m.mean[l][2];
+                const double* P = m.prec[l];
+                const double v0 = mul_add(P[2], d2, mul_add(P[0], d0, P[1] * d1));
+                const double v1 = mul_add(P[5], d2, mul_add(P[3], d0, P[4] * d1));
+                const double v2 = mul_add(P[8], d2, mul_add(P[6], d0, P[7] * d1));
+                const double D = mul_add(d2, v2, mul_add(d0, v0, d1 * v1));
+                const double t0 = mul_add(P[6], d2, mul_add(P[0], d0, P[3] * d1));
+                const double t1 = mul_add(P[7], d2, mul_add(P[1], d0, P[4] * d1));
+                const double t2 = mul_add(P[8], d2, mul_add(P[2], d0, P[5] * d1));
+                ng[0] = av * (v0 + t0); ng[1] = av * (v1 + t1); ng[2] = av * (v2 + t2);
+                ng[3] = REFINE ? D : D + 0.01;
+            }
+            if (l > 0) {
+                double o[4], q[4];
+                get(kD, l, o); get(kD, l - 1, q);
+                const double Al = o[3], dd = q[3], X = m.fX[l], Y = m.fY[l], Z = m.fZ[l];
+                const double n_dd = 1.0 - dd, n_av = 1.0 - av;
+                const double da = mul_add(X, dd, Y * n_dd) - Z * dd;
+                const double db = mul_add(Z, n_av, X * av - Y * av);
+                const double ya = Y * av * n_dd, yd = Y * n_dd, zd = Z * dd, zdn = zd * n_av, zn = Z * n_av, ad = av * dd;
+                const bool big = Al > 1e-12;
+                double fv[3], fs[3], fd[3], ga[3], gp[3];
+                blend_all3(m.mode[l], t, q, fv, fs, fd);
+                const double y = __drcp_rn(Al);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const double v = adj[c], s = t[c], cc = q[c];
+                    const double ds = mul_add(ad, fs[c], ya);
+                    const double dc = mul_add(ad, fd[c], zdn);
+                    const double pa = mul_add(fv[c], dd, yd * s) - zd * cc;
+                    const double pd = mul_add(zn, cc, fv[c] * av - Y * av * s);
+                    const double na = pa - o[c] * da, np = pd - o[c] * db;
+                    const double qa = quotient(na, Al, y), qp = quotient(np, Al, y), qs = quotient(ds, Al, y),
+                                 qc = quotient(dc, Al, y);
+                    ga[c] = v * (big ? qa : pa);
+                    gp[c] = v * (big ? qp : pd);
+                    ng[c] += v * (big ? qs : ds);
+                    adj[c] = v * (big ? qc : dc);
+                }
+                if constexpr (REFINE) {
+                    double ta = adj3 * da, tp = adj3 * db;
+                    ta += ga[0]; ta += ga[1]; ta += ga[2];
+                    tp += gp[0]; tp += gp[1]; tp += gp[2];
+                    ng[3] += ta;
+                    adj3 = tp;
+                } else {
+                    const double g3 = adj3 * da, p3 = adj3 * db;
+                    ng[3] += (ga[0] + ga[1]) + (ga[2] + g3);
+                    adj3 = (gp[0] + gp[1]) + (gp[2] + p3);
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) ng[c] += adj[c];
+                ng[3] += adj3;
+            }
+            put(kD, l, ng[0], ng[1], ng[2], ng[3]);
+        }
+        if (at_x) {
+#pragma unroll 1
+            for (int l = 0; l < L; ++l) {
+                double ng[4];
+                get(kD, l, ng);
+                put(kG, l, ng[0], ng[1], ng[2], ng[3]);
+            }
+            state = kLaneDir;
+            return;
+        }
+        double sy[NV], yy[NV], ya = 0.0;
+#pragma unroll
+        for (int c = 0; c < NV; ++c) { sy[c] = 0.0; yy[c] = 0.0; }
+#pragma unroll 1
+        for (int l = 0; l < L; ++l) {
+            double ng[4], g[4], s[4], yv[4] = {0.0, 0.0, 0.0, 0.0};
+            load_rec(ring(next, 0, l), s);
+            get(kD, l, ng); get(kG, l, g);
+#pragma unroll
+            for (int c = 0; c < NV; ++c) {
+                yv[c] = ng[c] - g[c];
+                sy[c] = mul_add(s[c], yv[c], sy[c]);
+                yy[c] = mul_add(yv[c], yv[c], yy[c]);
+            }
+            if (REFINE) { const double dy = ng[3] - g[3]; ya = mul_add(dy, dy, ya); }
+            store_rec(ring(next, 1, l), yv[0], yv[1], yv[2], yv[3]);
+            put(kG, l, ng[0], ng[1], ng[2], ng[3]);
+        }
+        double yyt = sum(yy);
+        if (REFINE) yyt += ya;
+        if (curvature(sum(sy), ss_kept, yyt)) {
+            next = next + 1 == kLaneRing ? 0 : next + 1;
+            valid = valid + 1 < kHistory ? valid + 1 : kHistory;
+        }
+        if (small_change) state = kLaneEnd;
+        else if (++it >= ctl.inner) state = kLaneEnd;
+        else state = kLaneDir;
+    }
+
+    // sy > 1e-9 sqrt(ss yy), sy > 0 and 1 / sy finite: by squares, except
+    // where rounding, under- or overflow could decide.
+    __device__ __forceinline__ static bool curvature(double sy, double ss, double yy) {
+        if (!(sy > 0.0)) return false;
+        const double t = 1e-18 * (ss * yy), r = sy * sy;
+        if (t > 1e-250 && t < 1e250 && r < 1e250 && fabs(r - t) > 1e-12 * t) return r > t;
+        return curvature_exact(sy, ss, yy);
+    }
+    __device__ __noinline__ static bool curvature_exact(double sy, double ss, double yy) {
+        return sy > 1e-9 * sqrt(ss * yy) && sy > 0.0 && isfinite(1.0 / sy);
+    }
+
+    // ---------------------------------------------------------- direction --
+    // Top of an inner iteration (kLaneDir: projected gradient test, two-loop
+    // direction) or the steepest-descent attempt (kLaneSteep).
+    __device__ __forceinline__ void direction() {
+        const bool steep = state == kLaneSteep;
+        uint32_t freem = 0;
+        {
+            double pg[NV];
+#pragma unroll
+            for (int c = 0; c < NV; ++c) pg[c] = 0.0;
+#pragma unroll 1
+            for (int l = 0; l < L; ++l) {
+                double x[4], g[4], v[4];
+                get(kX, l, x); get(kG, l, g);
+                v[3] = 0.0;
+#pragma unroll
+                for (int c = 0; c < NV; ++c) {
+                    const bool fr = !fixed_at(l, c, x[c], g[c]);
+                    freem |= fr ? 1u << (l * 4 + c) : 0u;
+                    v[c] = fr ? g[c] : 0.0;
+                    pg[c] = mul_add(v[c], v[c], pg[c]);
+                }
+                put(kD, l, v[0], v[1], v[2], v[3]);
+            }
+            if (!steep) {
+                count(2);
+                if (sum(pg) < 1e-16 || !isfinite(f)) { state = kLaneEnd; return; }
+            }
+        }
+        double q[L][4];
+#pragma unroll
+        for (int l = 0; l < L; ++l) get(kD, l, q[l]);
+        double scaling = 1.0;
+        bool have_scaling = false;
+        double2* coeff = slot(4 * L);
+#pragma unroll 1
+        for (int j = 0; j < valid; ++j) {
+            int k = next - 1 - j;
+            k = k < 0 ? k + kLaneRing : k;
+            double dot[NV], sy[NV], ss[NV], yy[NV];
+#pragma unroll
+            for (int c = 0; c < NV; ++c) { dot[c] = 0.0; sy[c] = 0.0; ss[c] = 0.0; yy[c] = 0.0; }
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+                double sv[4], yv[4];
+                load_rec(ring(k, 0, l), sv); load_rec(ring(k, 1, l), yv);
+#pragma unroll
+                for (int c = 0; c < NV; ++c)
+                    if (freem >> (l * 4 + c) & 1u) {
+                        dot[c] = mul_add(sv[c], q[l][c], dot[c]);
+                        sy[c] = mul_add(sv[c], yv[c], sy[c]);
+                        ss[c] = mul_add(sv[c], sv[c], ss[c]);
+                        yy[c] = mul_add(yv[c], yv[c], yy[c]);
+                    }
+            }
+            const double syt = sum(sy), yyt = sum(yy);
+            const double inv = curvature(syt, sum(ss), yyt) ? __drcp_rn(syt) : 0.0;
+            const double co = sum(dot) * inv;
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+                double yv[4];
+                load_rec(ring(k, 1, l), yv);
+#pragma unroll
+                for (int c = 0; c < NV; ++c)
+                    if (freem >> (l * 4 + c) & 1u) q[l][c] = mul_add(-co, yv[c], q[l][c]);
+            }
+            if (!have_scaling && inv > 0.0 && yyt > 0.0) { scaling = syt / yyt; have_scaling = true; }
+            coeff[j * kLaneBlock] = make_double2(co, inv);
+        }
+        scaling = fmax(1e-12, fmin(1e3, scaling));
+#pragma unroll
+        for (int l = 0; l < L; ++l)
+#pragma unroll
+            for (int c = 0; c < NV; ++c) q[l][c] *= scaling;
+#pragma unroll 1
+        for (int j = valid - 1; j >= 0; --j) {
+            int k = next - 1 - j;
+            k = k < 0 ? k + kLaneRing : k;
+            double dot[NV];
+#pragma unroll
+            for (int c = 0; c < NV; ++c) dot[c] = 0.0;
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+                double yv[4];
+                load_rec(ring(k, 1, l), yv);
+#pragma unroll
+                for (int c = 0; c < NV; ++c)
+                    if (freem >> (l * 4 + c) & 1u) dot[c] = mul_add(yv[c], q[l][c], dot[c]);
+            }
+            const double2 ci = coeff[j * kLaneBlock];
+            const double w = mul_add(-sum(dot), ci.y, ci.x);
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+                double sv[4];
+                load_rec(ring(k, 0, l), sv);
+#pragma unroll
+                for (int c = 0; c < NV; ++c)
+                    if (freem >> (l * 4 + c) & 1u) q[l][c] = mul_add(w, sv[c], q[l][c]);
+            }
+        }
+#pragma unroll
+        for (int l = 0; l < L; ++l) put(kD, l, q[l][0], q[l][1], q[l][2], q[l][3]);
+        double descent[NV];
+#pragma unroll
+        for (int c = 0; c < NV; ++c) descent[c] = 0.0;
+#pragma unroll 1
+        for (int l = 0; l < L; ++l) {
+            double x[4], g[4], d[4];
+            get(kX, l, x); get(kG, l, g); get(kD, l, d);
+#pragma unroll
+            for (int c = 0; c < NV; ++c) {
+                double v = -d[c];
+                if (fixed_bounds(l, c) || (x[c] <= 0.0 && v < 0.0) || (x[c] >= 1.0 && v > 0.0)) v = 0.0;
+                d[c] = v;
+                descent[c] = mul_add(v, g[c], descent[c]);
+            }
+            put(kD, l, d[0], d[1], d[2], d[3]);
+        }
+        if (!steep && !(sum(descent) < 0.0)) {
+            valid = 0; next = 0;
+#pragma unroll 1
+            for (int l = 0; l < L; ++l) {
+                double x[4], g[4], d[4];
+                get(kX, l, x); get(kG, l, g);
+                d[3] = 0.0;
+#pragma unroll
+                for (int c = 0; c < NV; ++c) d[c] = fixed_at(l, c, x[c], g[c]) ? 0.0 : -g[c];
+                put(kD, l, d[0], d[1], d[2], d[3]);
+            }
+        }
+        second = steep;
+        bt = 0;
+        step = 1.0;
+        state = kLaneTrial;
+    }
+
+    // -------------------------------------------------------- outer steps --
+    // End of an outer step (kLaneEnd): multipliers, penalty, and the next
+    // outer step (true), or the next start / the pixel's result.
+    enum : int { kNextOuter, kNextStart, kFinished };
+    __device__ __forceinline__ int end_outer() {
+        const double tol2 = ctl.outer_tolerance * ctl.outer_tolerance;
+        double nn[NV], mo[NV];
+#pragma unroll
+        for (int c = 0; c < NV; ++c) { nn[c] = resx[c] * resx[c]; mo[c] = 0.0; }
+        const double norm = sum(nn);
+        const bool feasible = norm < tol2;
+#pragma unroll
+        for (int c = 0; c < NV; ++c) lam[c] = mul_add(-rho, resx[c], lam[c]);
+        if (norm > 0.0625 * oldnorm) rho *= 10.0;
+#pragma unroll 1
+        for (int l = 0; l < L; ++l) {
+            double x[4], o[4];
+            load_rec(ox_rec(l), o);
+            get(kX, l, x);
+#pragma unroll
+            for (int c = 0; c < NV; ++c) { const double dl = x[c] - o[c]; mo[c] = mul_add(dl, dl, mo[c]); }
+        }
+        const double motion = sum(mo);
+        frozen = (motion == 0.0 && !best_moved) ? frozen + 1 : 0;
+        if (ctl.frozen_stop > 0 && frozen >= ctl.frozen_stop) {
+            if (start + 1 < ctl.starts) { ++start; return kNextStart; }
+            return kFinished;
+        }
+        if (!(motion < tol2 && feasible) && outer + 1 < ctl.outer) { ++outer; return kNextOuter; }
+        if (start + 1 < ctl.starts) { ++start; return kNextStart; }
+        return kFinished;
+    }
+
+    __device__ __forceinline__ void begin_outer() {
+        count(4);
+#pragma unroll 1
+        for (int l = 0; l < L; ++l) {
+            double x[4];
+            get(kX, l, x);
+            store_rec(ox_rec(l), x[0], x[1], x[2], x[3]);
+        }
+        best_moved = false;
+        state = kLaneOuter;
+    }
+
+    __device__ __forceinline__ double pinned_alpha(int l) const {
+        return (a.opaque && l == 0) ? 1.0 : a.targets[size_t(l) * size_t(a.n) + pixel];
+    }
+    __device__ __forceinline__ double background(int c) const { return a.targets[(size_t(L) + c) * size_t(a.n) + pixel]; }
+
+    // The start-0 seed of component c of layer l.
+    __device__ __forceinline__ double seed(int l, int c) const {
+        const size_t i = size_t(pixel);
+        if constexpr (REFINE) {
+            if (c == 3) return pinned_alpha(l);
+            return (a.smooth && l == 0) ? background(c) : a.first[(size_t(l) * size_t(a.n) + i) * 4 + c];
+        } else {
+            const float* wp;
+            if constexpr (BATCH) wp = a.jobs[job_id].warm; else wp = a.warm;
+            if (wp) return double(wp[i * size_t(4 * L) + (c == 3 ? l : L + 3 * l + c)]);
+            if (c == 3) return (a.opaque && l == 0) ? 1.0 : 0.5;
+            return fmin(1.0, fmax(0.0, models_->mean[l][c]));
+        }
+    }
+
+    // Bounds of component c of layer l applied to v.
+    __device__ __forceinline__ double clamp_bounds(int l, int c, double v) const {
+        if (REFINE && c == 3) return v;
+        double lo = 0.0, hi = 1.0;
+        if (l == 0 && c == 3 && a.opaque) lo = 1.0;
+        if (REFINE && l == 0 && c != 3 && a.smooth) lo = hi = background(c);
+        return v < lo ? lo : (v > hi ? hi : v);
+    }
+
+    // Component c of layer l of x in shared memory.
+    __device__ __forceinline__ double* x_at(int l, int c) const {
+        return reinterpret_cast<double*>(slot(kX * 2 * L + 2 * l + (c >> 1))) + (c & 1);
+    }
+
+    // Starting point `start` (one component at a time: rare, so kept small).
+    __device__ __forceinline__ void begin_start() {
+        const Models<double>& m = *models_;
+        const int s = start;
+#pragma unroll 1
+        for (int k = 0; k < 4 * L; ++k) {
+            const int l = k >> 2, c = k & 3;
+            double v = seed(l, c);
+            if (s == 1) {
+                if (c != 3) v = (!REFINE && l == 0) ? fmin(1.0, fmax(0.0, image()[3 * size_t(pixel) + c])) : m.mean[l][c];
+                else if (!REFINE) v = l == 0 ? 1.0 : 0.0;
+            } else if (s == 2) {
+                if (c != 3) v = fmax(0.05, fmin(0.95, m.mean[l][c]));
+                else if (!REFINE) v = 0.5;
+            }
+            *x_at(l, c) = clamp_bounds(l, c, v);
+        }
+        if (s == 2) {
+            // Move Dodge/Burn sources into the unsaturated branch.
+#pragma unroll 1
+            for (int c = 0; c < 3; ++c) {
+                double da = *x_at(0, 3), dest = *x_at(0, c);
+#pragma unroll 1
+                for (int l = 1; l < L; ++l) {
+                    const double al = *x_at(l, 3), X = m.fX[l], Y = m.fY[l], Z = m.fZ[l];
+                    const double Al = X * al * da + Y * al * (1.0 - da) + Z * da * (1.0 - al);
+                    double sv = *x_at(l, c);
+                    if (dest >= 0.0 && dest <= 1.0 && m.mode[l] == 6) sv = fmin(sv, fmax(0.0, 1.0 - dest - 0.05));
+                    if (dest >= 0.0 && dest <= 1.0 && m.mode[l] == 7) sv = fmax(sv, fmin(1.0, 1.0 - dest + 0.05));
+                    sv = clamp_bounds(l, c, sv);
+                    *x_at(l, c) = sv;
+                    const double pre = blend_value_call<double>(m.mode[l], sv, dest) * al * da +
+                                       Y * al * (1.0 - da) * sv + Z * da * (1.0 - al) * dest;
+                    dest = Al > 1e-12 ? pre / Al : pre;
+                    da = Al;
+                }
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < NV; ++c) lam[c] = 0.0;
+        rho = 100.0;
+        outer = 0;
+        frozen = 0;
+    }
+
+    // ------------------------------------------------------------- pixels --
+    // Writes the finished pixel: output (pinned values exactly), status, miss
+    // list. The point written is the best point, whose constraint norm is
+    // best_norm (the same operations on the same values as a check of the
+    // written point); a pixel without one writes its seed, checked here.
+    __device__ __forceinline__ void store(bool skipped) {
+        const size_t n = pixels(), i = size_t(pixel);
+        double* outp;
+        int32_t* stp;
+        if constexpr (BATCH) { outp = a.jobs[job_id].out; stp = a.jobs[job_id].status; }
+        else { outp = a.out; stp = a.status; }
+#pragma unroll 1
+        for (int k = 0; k < 4 * L; ++k) {
+            const int l = k >> 2, c = k & 3;
+            double v = have_best ? best_rec(l)[c] : seed(l, c);
+            if (REFINE && c == 3) v = pinned_alpha(l);
+            if (REFINE && c != 3 && l == 0 && a.smooth) v = background(c);
+            if (!REFINE && c == 3 && l == 0 && a.opaque) v = 1.0;
+            outp[(size_t(l) * n + i) * 4 + c] = v;
+        }
+        if (skipped) {
+            if (stp) stp[i] = 8;
+            if (a.input_failed) atomicAdd(a.input_failed, 1);
+            return;
+        }
+        if (!have_best) best_norm = written_norm(*models_, outp, image() + 3 * i, n, i);
+        const bool miss = !(best_norm < ctl.outer_tolerance * ctl.outer_tolerance);
+        if (stp) stp[i] = miss ? 3 : 0;
+        if (miss && a.miss_list) a.miss_list[atomicAdd(a.miss_count, 1)] = int32_t(gidx);
+    }
+
+    // Constraint norm of the written point, one channel at a time.
+    __device__ __noinline__ static double written_norm(const Models<double>& m, const double* outp, const double* rgb,
+                                                       size_t n, size_t i) {
+        double total = 0.0, A = 0.0, first_two = 0.0;
+#pragma unroll 1
+        for (int c = 0; c < 3; ++c) {
+            double cc = 0.0;
+#pragma unroll 1
+            for (int l = 0; l < L; ++l) {
+                const double* o = outp + (size_t(l) * n + i) * 4;
+                const double sv = o[c], al = o[3];
+                if (l == 0) { A = al; cc = sv; continue; }
+                const double dd = A, X = m.fX[l], Y = m.fY[l], Z = m.fZ[l];
+                const double Al = X * al * dd + Y * al * (1.0 - dd) + Z * dd * (1.0 - al);
+                const double pre = blend_value<double>(m.mode[l], sv, cc) * al * dd + Y * al * (1.0 - dd) * sv +
+                                   Z * dd * (1.0 - al) * cc;
+                cc = Al > 1e-12 ? pre / Al : pre;
+                A = Al;
+            }
+            const double r = cc - rgb[c];
+            if (c == 0) first_two = r * r;
+            else if (c == 1) first_two += r * r;
+            else total = r * r;
+        }
+        if (!REFINE) total += (A - 1.0) * (A - 1.0);
+        return first_two + total;
+    }
+
+    // Loads the pixel of queue entry `job`; false when it is written without
+    // a solve (refinement targets that cannot be normalized).
+    __device__ __forceinline__ bool load(int job) {
+        gidx = a.list ? a.list[job] : (a.order ? a.order[job] : a.first_pixel + job);
+        int i = gidx;
+        if constexpr (BATCH) {
+            int lo = 0, hi = a.job_count - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (a.jobs[mid].offset <= int64_t(gidx)) lo = mid; else hi = mid - 1;
+            }
+            job_id = lo;
+            models_ = static_cast<const Models<double>*>(a.models) + a.jobs[lo].model;
+            i = gidx - int(a.jobs[lo].offset);
+        }
+        pixel = i;
+        const double* p = image() + 3 * size_t(i);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) target[c] = p[c];
+        have_best = false;
+        best_norm = INFINITY; best_energy = INFINITY;
+        if (a.counters)
+#pragma unroll
+            for (int k = 0; k < 5; ++k) a.counters[5 * size_t(gidx) + k] = 0;
+        start = 0;
+        return !(REFINE && a.input_status && a.input_status[i] != 0);
+    }
+
+    // --------------------------------------------------------------- loop --
+    __device__ void run() {
+        const unsigned full = 0xffffffffu;
+        const int total = a.list ? min(*a.list_count, a.list_limit) : (a.pixel_count >= 0 ? a.pixel_count : a.n);
+        // A small launch spreads its pixels over all warps.
+        const int warps = int(gridDim.x) * (kLaneBlock / 32);
+        if (total <= 0 || lane > (total - 1) / warps) state = kLaneIdle;
+        for (;;) {
+            const int live = __syncthreads_count(state != kLaneIdle);
+            if (live == 0) break;
+            const int ne = __syncthreads_count(state == kLaneEnd || state == kLaneFetch);
+            int nf = __syncthreads_count(state == kLaneTrial || state == kLaneOuter);
+            if (ne > 0 && (8 * ne >= kOuterQuorum * live || nf == 0)) {
+                int what = kFinished;
+                bool write = false, skipped = false;
+                if (state == kLaneEnd) {
+                    what = end_outer();
+                    write = what == kFinished;
+                }
+                // Finished pixels are written, and the lanes without a pixel
+                // take the next queue entries together.
+                for (;;) {
+                    if (write) { store(skipped); write = false; state = kLaneFetch; }
+                    const unsigned want = __ballot_sync(full, state == kLaneFetch);
+                    if (want == 0) break;
+                    const int leader = __ffs(want) - 1;
+                    int base = 0;
+                    if (lane == leader) base = int(atomicAdd(a.queue, unsigned(__popc(want))));
+                    base = __shfl_sync(full, base, leader);
+                    if (state == kLaneFetch) {
+                        const int job = base + __popc(want & ((1u << lane) - 1u));
+                        if (job >= total) state = kLaneIdle;
+                        else {
+                            state = kLaneEnd;
+                            what = kNextStart;
+                            if (!load(job)) write = skipped = true;
+                        }
+                    }
+                }
+                if (state == kLaneEnd) {
+                    if (what == kNextStart) begin_start();
+                    begin_outer();
+                }
+            }
+            __syncwarp();
+            nf = __syncthreads_count(state == kLaneTrial || state == kLaneOuter);
+            const int nd = __syncthreads_count(state == kLaneDir || state == kLaneSteep);
+            if (nd > 0 && (8 * nd >= kDirectionQuorum * live || nf == 0)) {
+                if (state == kLaneDir || state == kLaneSteep) direction();
+                __syncwarp();
+            }
+            nf = __syncthreads_count(state == kLaneTrial || state == kLaneOuter);
+            const int nb = __syncthreads_count(state == kLaneGrad);
+            const bool gradients = nb > 0 && (8 * nb >= kGradientQuorum * live || nf == 0);
+            if (state == kLaneTrial || state == kLaneOuter || (gradients && state == kLaneGrad)) {
+                const bool mine = state == kLaneGrad;
+                forward();
+                pending = mine;
+            }
+            __syncwarp();
+            if (gradients) {
+                if (pending) backward();
+                pending = false;
+                __syncwarp();
+            }
+        }
+        if (a.tally) {
+            const uint32_t v = __reduce_add_sync(full, n_value), g = __reduce_add_sync(full, n_grad);
+            if (lane == 0) {
+                atomicAdd(a.tally + 0, (unsigned long long)v);
+                atomicAdd(a.tally + 1, (unsigned long long)g);
+            }
+        }
+    }
+};
+
+template <int L, bool REFINE, bool BATCH>
+__global__ void __launch_bounds__(kLaneBlock, lane_blocks_per_sm(L))
+solve_lanes(const __grid_constant__ Models<double> m, const __grid_constant__ SolverControls ctl,
+            const __grid_constant__ SolveArgs a) {
+    LaneSolver<L, REFINE, BATCH> solver(&m, ctl, a);
+    solver.run();
+}
+
+}  // namespace unb

@@ -27,6 +27,8 @@ cudaError_t launch_solve_fp32(int L, bool refine, int variant, const Models<floa
 
 cudaError_t launch_solve_fp64(int L, bool refine, int variant, const Models<double>& m, const SolverControls& c,
                               const SolveArgs& a, int threads, int sms, cudaStream_t s) {
+    if (variant == kFp64Lanes)
+        return by_layers(L, [&](auto k) { return solve_lanes_layers<decltype(k)::value>(refine, false, m, c, a, sms, s); });
     return by_layers(L, [&](auto k) { return solve_fp64_layers<decltype(k)::value>(refine, variant, m, c, a, threads, sms, s); });
 }
 
@@ -37,6 +39,10 @@ cudaError_t launch_solve_batch_fp32(int L, int variant, const SolverControls& c,
 
 cudaError_t launch_solve_batch_fp64(int L, int variant, const SolverControls& c, const SolveArgs& a, int threads,
                                     int sms, cudaStream_t s) {
+    if (variant == kFp64Lanes)
+        return by_layers(L, [&](auto k) {
+            return solve_lanes_layers<decltype(k)::value>(false, true, Models<double>{}, c, a, sms, s);
+        });
     return by_layers(L, [&](auto k) { return solve_batch_fp64_layers<decltype(k)::value>(variant, c, a, threads, sms, s); });
 }
 

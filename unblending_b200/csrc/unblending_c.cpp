@@ -452,6 +452,19 @@ int fp64_variant(const unblending_solver_options& so, bool refine) {
     return so.fp64_variant >= 0 ? so.fp64_variant : default_fp64_variant(refine);
 }
 
+// Whether an FP64 solve of up to `count` pixels runs one pixel per lane
+// (lane_solver.cuh) rather than on quads: by default, unless the caller names
+// a quad variant or a block size. A first pass of up to three layers and fewer
+// than 32,768 pixels stays on quads: there the last pixels' serial chain
+// decides, and a quad's evaluation is the shorter one (three layers, first
+// pass, lanes / quads in ms: 5,184 pixels 2.4 / 2.0, 16,384 2.4 / 1.9, 30,976
+// 3.0 / 2.6, 65,536 3.3 / 4.0; refinement 2.5 / 3.0, 2.8 / 3.4, 2.8 / 3.1, 3.2 /
+// 4.5; five layers, first pass: 576 pixels 3.2 / 4.8, 16,384 5.3 / 5.6, 65,536
+// 7.2 / 12.7; eight layers, 576 4.2 / 9.1, 65,536 14 / 57).
+bool lane_solve(const unblending_solver_options& so, int L, bool refine, int64_t count) {
+    return so.fp64_variant < 0 && so.threads_per_block == 0 && (refine || L > 3 || count >= 32768);
+}
+
 // Bytes of a global-memory L-BFGS history array for L layers and values of
 // `elem` bytes, sized for kGlobalHistoryBlocksPerSm blocks on every SM.
 size_t history_lanes(int sms) { return size_t(kGlobalHistoryBlocksPerSm) * sms * kSliceStride; }
@@ -465,6 +478,11 @@ void attach_history(SolveArgs& a, void* array, bool fp64, int variant, int sms) 
     if (!variant_global_history(fp64, variant)) return;
     a.history = array;
     a.history_lanes = int(history_lanes(sms));
+}
+// The same for the lane kernels (`array` of lane_history_bytes(L, sms) bytes).
+void attach_lane_history(SolveArgs& a, void* array, int L, int sms) {
+    a.history = array;
+    a.history_lanes = lane_blocks(L, sms) * kLaneBlock;
 }
 
 SolverControls controls(const unblending_solver_options& so) {
@@ -521,6 +539,7 @@ template <class T> Models<T> make_models(const unblending_layer* layers, int L) 
         for (int k = 0; k < 9; ++k) m.prec[l][k] = T(layers[l].precision[k]);
         m.mode[l] = layers[l].blend_mode;
         m.X[l] = layers[l].comp_x; m.Y[l] = layers[l].comp_y; m.Z[l] = layers[l].comp_z;
+        m.fX[l] = T(m.X[l]); m.fY[l] = T(m.Y[l]); m.fZ[l] = T(m.Z[l]);
         set_blend_table(m, l, layers[l].blend_mode);
     }
     return m;
@@ -666,12 +685,17 @@ PassResult enqueue_pass(Context& c, const Spec& sp, bool refine, const unblendin
     const int threads = so.threads_per_block ? so.threads_per_block : 128;
     // One history array serves the FP32 solve and the FP64 re-solve (they run
     // one after the other on the stream).
-    void* history = c.history.get<unsigned char>(history_bytes(L, sizeof(double), c.sms));
+    const int solved = io.pixel_count >= 0 ? io.pixel_count : int(n);
+    const bool lanes = lane_solve(so, L, refine, solved);
+    const int v64 = lanes ? kFp64Lanes : fp64_variant(so, refine);
+    // (the FP32 solve's global history, where its variant has one, is of the quads' size)
+    const size_t quad_history = lanes && so.precision == UNBLENDING_PRECISION_FP64 ? 0 : history_bytes(L, sizeof(double), c.sms);
+    void* history = c.history.get<unsigned char>(std::max(quad_history, lanes ? lane_history_bytes(L, c.sms) : 0));
     if (so.precision == UNBLENDING_PRECISION_FP64) {
-        attach_history(a, history, true, fp64_variant(so, refine), c.sms);
+        if (lanes) attach_lane_history(a, history, L, c.sms);
+        else attach_history(a, history, true, v64, c.sms);
         const Range range(refine ? "refinement solve (fp64)" : "first-pass solve (fp64)");
-        const int solved = io.pixel_count >= 0 ? io.pixel_count : int(n);
-        if (so.defer_outer > 0 && solved > 0 && variant_defers(fp64_variant(so, refine), refine)) {
+        if (so.defer_outer > 0 && solved > 0 && variant_defers(v64, refine)) {
             // Pixels still unsolved at outer step defer_outer leave this
             // launch (up to a quarter of its pixels; the rest carry on) ...
             a.defer_outer = so.defer_outer;
@@ -680,8 +704,7 @@ PassResult enqueue_pass(Context& c, const Spec& sp, bool refine, const unblendin
             a.defer_count = reinterpret_cast<int32_t*>(queues + 3);
             a.defer_state = c.defer_state.get<double>(size_t(a.defer_capacity) * 4 * size_t(defer_words(L)));
         }
-        ck(launch_solve_fp64(L, refine, fp64_variant(so, refine), make_models<double>(layers, L), ctl, a, threads,
-                             c.sms, s));
+        ck(launch_solve_fp64(L, refine, v64, make_models<double>(layers, L), ctl, a, threads, c.sms, s));
         ++t_launches;
         if (a.defer_outer > 0) {
             // ... and are resumed together by the next launch (queue 2), from
@@ -693,8 +716,7 @@ PassResult enqueue_pass(Context& c, const Spec& sp, bool refine, const unblendin
             d.order = nullptr;
             d.queue = queues + 2;
             d.input_status = nullptr; d.input_failed = nullptr;
-            ck(launch_solve_fp64(L, refine, fp64_variant(so, refine), make_models<double>(layers, L), ctl, d, threads,
-                                 c.sms, s));
+            ck(launch_solve_fp64(L, refine, v64, make_models<double>(layers, L), ctl, d, threads, c.sms, s));
             ++t_launches;
             a.defer_outer = 0;
         }
@@ -708,8 +730,7 @@ PassResult enqueue_pass(Context& c, const Spec& sp, bool refine, const unblendin
             b.queue = queues + 1;
             b.input_status = nullptr; b.input_failed = nullptr;
             b.warm = nullptr;
-            ck(launch_solve_fp64(L, refine, fp64_variant(so, refine), make_models<double>(layers, L), ctl, b, threads,
-                                 c.sms, s));
+            ck(launch_solve_fp64(L, refine, v64, make_models<double>(layers, L), ctl, b, threads, c.sms, s));
             ++t_launches;
         } else {
             ck(cudaMemcpyAsync(counts + 1, counts + 0, sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
@@ -753,9 +774,9 @@ PassResult enqueue_pass(Context& c, const Spec& sp, bool refine, const unblendin
             b.warm = nullptr;   // the reference's (cold) start
             b.history = nullptr; b.history_lanes = 0;
             b.tally = R.tally;
-            attach_history(b, history, true, fp64_variant(so, refine), c.sms);
-            ck(launch_solve_fp64(L, refine, fp64_variant(so, refine), make_models<double>(layers, L), ctl_re, b,
-                                 threads, c.sms, s));
+            if (lanes) attach_lane_history(b, history, L, c.sms);
+            else attach_history(b, history, true, v64, c.sms);
+            ck(launch_solve_fp64(L, refine, v64, make_models<double>(layers, L), ctl_re, b, threads, c.sms, s));
             ++t_launches;
         } else {
             ck(cudaMemcpyAsync(counts + 1, counts + 0, sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
