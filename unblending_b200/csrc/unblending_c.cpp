@@ -1094,6 +1094,7 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
                 std::vector<std::pair<int, float*>> infer;   // job, warm slice
                 MlpDevice net;
                 int variant = 0, threads = 128;
+                int v64 = 0;                // FP64 kernel of the group's solve or re-solve
                 int64_t total = 0;
                 int32_t* order = nullptr;   // colour order of the group's queue (pixel_order)
                 uint32_t* order_cells = nullptr;
@@ -1194,7 +1195,15 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
                 if (so.precision == UNBLENDING_PRECISION_FP64 && G.infer.empty()) a.miss_count = G.counts + 1;
                 plan->counts.push_back(G.counts);
                 plan->pixels += total;
-                void* history = plan->alloc<unsigned char>(history_bytes(L, sizeof(double), c.sms));
+                const bool lanes = lane_solve(so, L, false, total);
+                G.v64 = lanes ? kFp64Lanes : fp64_variant(so, false);
+                const size_t quad_history =
+                    lanes && so.precision == UNBLENDING_PRECISION_FP64 ? 0 : history_bytes(L, sizeof(double), c.sms);
+                void* history = plan->alloc<unsigned char>(std::max(quad_history, lanes ? lane_history_bytes(L, c.sms) : 0));
+                auto attach_fp64 = [&](SolveArgs& x) {
+                    if (lanes) attach_lane_history(x, history, L, c.sms);
+                    else attach_history(x, history, true, G.v64, c.sms);
+                };
                 // Autotuner: time each FP32 kernel variant / block size on a
                 // sample of this group's pixels spread over its images.
                 const auto tkey = std::make_pair(L, so.precision);
@@ -1232,10 +1241,10 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
                     G.variant = so.kernel_variant >= 0 ? so.kernel_variant : default_fp32_variant(L, false);
                     G.threads = so.threads_per_block ? so.threads_per_block : 128;
                 }
-                if (so.precision == UNBLENDING_PRECISION_FP64) attach_history(a, history, true, fp64_variant(so, false), c.sms);
+                if (so.precision == UNBLENDING_PRECISION_FP64) attach_fp64(a);
                 else attach_history(a, history, false, G.variant, c.sms);
                 attach_history(G.mid, history, false, G.variant, c.sms);
-                attach_history(b, history, true, fp64_variant(so, false), c.sms);
+                attach_fp64(b);
                 gs.push_back(G);
             }
             // Capture every group's work into one graph, each group on its own
@@ -1276,10 +1285,10 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
                         ++launches;
                     }
                     if (so.precision == UNBLENDING_PRECISION_FP64) {
-                        ck(launch_solve_batch_fp64(G.L, fp64_variant(so, false), ctl, G.fp, 128, c.sms, s));
+                        ck(launch_solve_batch_fp64(G.L, G.v64, ctl, G.fp, 128, c.sms, s));
                         ++launches;
                         if (!G.infer.empty()) {
-                            ck(launch_solve_batch_fp64(G.L, fp64_variant(so, false), ctl, G.re, 128, c.sms, s));
+                            ck(launch_solve_batch_fp64(G.L, G.v64, ctl, G.re, 128, c.sms, s));
                             ++launches;
                         }
                     } else {
@@ -1290,7 +1299,7 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
                             ++launches;
                         }
                         if (so.resolve_misses) {
-                            ck(launch_solve_batch_fp64(G.L, fp64_variant(so, false), ctl_re, G.re, 128, c.sms, s));
+                            ck(launch_solve_batch_fp64(G.L, G.v64, ctl_re, G.re, 128, c.sms, s));
                             ++launches;
                         } else {
                             ck(cudaMemcpyAsync(G.counts + 1, G.counts, sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
