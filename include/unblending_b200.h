@@ -50,9 +50,8 @@ typedef struct unblending_solver_options {
                                    Pixels the learned start leaves unsolved get the plain solve from the
                                    reference's start (FP64 precision: the FP64 solve; FP32 precision with
                                    resolve_misses: the FP32 solve, and what that misses the FP64 re-solve). */
-    int32_t fp64_variant;       /* FP64 solve and re-solve: -1 default, one pixel per lane (first passes of up to
-                                   three layers and fewer than 32,768 pixels, and calls that set
-                                   threads_per_block, run the quad kernels 3 and 7). Quad kernels (four or three
+    int32_t fp64_variant;       /* FP64 solve and re-solve: -1 default, one pixel per lane (calls that set
+                                   threads_per_block run the quad kernels 3 and 7). Quad kernels (four or three
                                    lanes per pixel), history in shared memory with 0 uncapped registers, 1 capped for 2 blocks per SM; 2 history in global memory,
                                    x/g/d in shared memory, evaluation rolled, 3 blocks per SM; 3 as 2 with the
                                    start and bounds in global memory, 4 blocks per SM; 4/5 as 3/2 with three

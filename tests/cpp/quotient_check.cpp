@@ -50,6 +50,16 @@ int main() {
         check(make(significand(int(next() % 8)), int(next() % 80) - 78), b);
     }
     check(0.0, 0.75);
+    // The reciprocal from approximations good to 2^-20 (either side).
+    for (int i = 0; i < 4000000; ++i) {
+        const double b = make(significand(int(next() % 8)), int(next() % 280) - 39);
+        uint64_t u;
+        std::memcpy(&u, &b, 8);
+        if ((u & 0xFFFFFFFFFFFFFull) == 0xFFFFFFFFFFFFFull) continue;   // (all ones: set by its bits)
+        const double r = 1.0 / b, y = unb::refine_reciprocal(b, r * (1.0 + (double(next() % 2001) - 1000.0) * 0x1p-30));
+        ++tried;
+        if (y != r) ++differ;
+    }
     std::printf("%ld of %ld\n", differ, tried);
     return differ ? 1 : 0;
 }

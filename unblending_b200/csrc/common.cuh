@@ -72,14 +72,17 @@ struct SolverControls {
 // A lane's global-memory records (32 bytes: one layer's three colours and
 // alpha) are the steps and gradient changes of the L-BFGS ring, which has a
 // spare slot that an accepted step fills before its curvature test, the best
-// point, and the outer step's start.
+// point, the outer step's start, and two of what an outer step keeps.
 constexpr int kLaneBlock = 128;
 constexpr int kLaneRing = kHistory + 1;
-__host__ __device__ constexpr int lane_records(int L) { return (2 * kLaneRing + 2) * L; }
+__host__ __device__ constexpr int lane_records(int L) { return (2 * kLaneRing + 2) * L + 2; }
 // Shared memory of a lane in 16-byte units: x, g, d (4 L values each; d's area
 // also takes the two-loop recursion's coefficients, six pairs).
 __host__ __device__ constexpr int lane_smem_units(int L) { return 4 * L + (2 * L > kHistory ? 2 * L : kHistory); }
-__host__ __device__ constexpr int lane_smem_bytes(int L) { return lane_smem_units(L) * kLaneBlock * 16; }
+__host__ __device__ constexpr bool lane_shared_targets(int L) { return L != 6; }
+__host__ __device__ constexpr int lane_smem_bytes(int L) {
+    return lane_smem_units(L) * kLaneBlock * 16 + (lane_shared_targets(L) ? 7 * kLaneBlock * 8 : 0);
+}
 // Resident blocks per SM: what shared memory holds for many layers (61 KB a
 // block at five layers, 98 KB at eight), and enough registers for the
 // direction's unrolled loops for few (a third block more at five layers, 128

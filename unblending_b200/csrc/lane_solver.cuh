@@ -21,10 +21,17 @@
 // actions as phases, all warps at once: every trip evaluates the lanes with a
 // trial, and the other actions run when a share of the block's lanes waits
 // for them (or none has a trial). With each warp on its own schedule, the
-// instruction cache thrashed between the phases' code (85 KB; 4 to 7 cycles
+// instruction cache thrashed between the phases' code (85-100 KB; 4 to 7 cycles
 // of fetch stall per issue, 75 + 45 ms for the two passes of the 1024x1024
-// five-layer image); with the block in phase the stall is 0.14 cycles (51 + 29
-// ms, against 134 + 99 on quads).
+// five-layer image); with the block in phase the stall is 0.3 cycles (42 + 23
+// ms, against 134 + 99 on quads). Even a block whose warps meet once a trip
+// only is slower (46 + 28 ms).
+//
+// What bounds it (1024x1024, five layers, first pass): latency at three warps
+// per scheduler (the shared memory and registers that a pixel's state and the
+// direction's loops take) and lanes that wait for a phase: 43 % of issue slots,
+// 38 % of the FP64 pipe, 13.5 of 32 lanes active. Trials take 42 % of the time,
+// directions 30 %, gradients 13 %, the meetings 15 %, outer steps 3 %.
 //
 // An accepted trial needs its gradient once; the lane's values repeat their
 // evaluation during the next trial phase, beside the lanes that evaluate
@@ -36,6 +43,18 @@
 #include "solver.cuh"
 
 namespace unb {
+
+// RN(1/b) from the hardware's approximation, without the branch to a slow path
+// that __drcp_rn takes, so that it overlaps the code around it (with
+// __drcp_rn the two passes of the 1024x1024 five-layer image took 1.03 times as
+// long).
+__device__ __forceinline__ double reciprocal(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = refine_reciprocal(b, y);
+    const bool ones = (uint32_t(__double2hiint(b)) | 0xfff00000u) == 0xffffffffu && __double2loint(b) == -1;
+    return __hiloint2double(__double2hiint(y), ones ? 1 : __double2loint(y));
+}
 
 __device__ __forceinline__ double mul_add(double a, double b, double c) { return __dadd_rn(__dmul_rn(a, b), c); }
 
@@ -77,7 +96,7 @@ __device__ __forceinline__ void blend_value3(int mode, const double* s, const do
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const double p = mode == 6 ? d[c] : 1.0 - d[c], q = mode == 6 ? 1.0 - s[c] : s[c];
-            const double v = quotient(p, q, __drcp_rn(q));
+            const double v = quotient(p, q, reciprocal(q));
             const double r = p < eps ? 0.0 : (q < eps ? 1.0 : (v < 1.0 ? v : 1.0));
             f[c] = mode == 6 ? r : 1.0 - r;
         }
@@ -117,8 +136,8 @@ __device__ __forceinline__ void blend_all3(int mode, const double* s, const doub
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const double p = mode == 6 ? d[c] : 1.0 - d[c], q = mode == 6 ? 1.0 - s[c] : s[c];
-            const double y = __drcp_rn(q), qq = q * q;
-            const double v = quotient(p, q, y), g = quotient(p, qq, __drcp_rn(qq));
+            const double y = reciprocal(q), qq = q * q;
+            const double v = quotient(p, q, y), g = quotient(p, qq, reciprocal(qq));
             const bool dark = p < eps, flat = dark || q < eps || 1.0 < v;
             const double r = dark ? 0.0 : (flat ? 1.0 : v);
             f[c] = mode == 6 ? r : 1.0 - r;
@@ -207,74 +226,114 @@ extern __shared__ __align__(16) unsigned char lane_smem[];
 
 // Eighths of a block's live lanes that start a phase: the end of an outer
 // step, a direction, a gradient. Measured on the 1024x1024 five-layer image,
-// first pass + refinement in ms: 4, 2, 2: 50.8 + 29.2; 2, 2, 2: 52.6 + 29.8; 4, 3,
-// 2: 52.5 + 32.6; 4, 2, 3: 49.6 + 30.4; 3, 1, 2: 53.9 + 29.6.
-constexpr int kOuterQuorum = 4, kDirectionQuorum = 2, kGradientQuorum = 2;
+// first pass + refinement in ms: 2, 2, 2: 42.1 + 26.5; 4, 2, 2: 41.5 + 27.1; 1.5, 2, 2:
+// 42.8 + 27.0; 1.5, 1.5, 1.5: 44.8 + 27.6; 1.5, 3, 3: 42.2 + 27.7; 1, 1, 1: 49.2 + 30.1.
+constexpr int kOuterQuorum = 2, kDirectionQuorum = 2, kGradientQuorum = 2;
 enum : int { kLaneIdle = 0, kLaneTrial, kLaneOuter, kLaneGrad, kLaneDir, kLaneSteep, kLaneEnd, kLaneFetch };
 
 template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     static constexpr int NV = REFINE ? 3 : 4;    // components of a layer that the method moves
+    static constexpr bool kSharedTargets = lane_shared_targets(L);
     const Models<double>* models_;
     const SolverControls& ctl;
     const SolveArgs& a;
     const int lane = threadIdx.x & 31;
-    double* rec_base;
-    size_t rec_stride;      // doubles between a lane's records
-    int job_id = -1;
+    double* rec_base;       // this lane's records, kLaneBlock apart: a block's are contiguous
     uint32_t n_value = 0, n_grad = 0;
 
-    // Pixel.
-    int state = kLaneFetch, pixel = 0, gidx = 0;
-    double target[3];
-    double lam[NV], resx[NV];
-    double rho, f, oldnorm, step, best_norm, best_energy, ss_kept;
-    int start, outer, it, bt, valid, next, frozen;
+    // The pixel's state that its trials read. The rest, read once an outer
+    // step, is in two records: the constraint residual at x, and `Outer`.
+    int state = kLaneFetch;
+    double target_[kSharedTargets ? 1 : 3], lam_[kSharedTargets ? 1 : NV];
+    double rho, f, step, best_norm, best_energy;
+    double best_step;   // kBestAtTrial: its step along d
+    int it, bt, valid, next;
     bool second;        // the line search's steepest-descent attempt
     bool from_trial;    // kLaneGrad: the point is an accepted trial (else the outer step's start)
-    bool small_change, best_moved, have_best;
-    bool pending = false;   // this trip computes the gradient
+    bool small_change, best_moved;
+    // Where the best point is: nowhere yet, in its records, x itself, or the
+    // trial point of step best_step. It is written to its records when x or d
+    // is about to change and it would be lost: most accepted points are better
+    // than the one before, so most best points never are (a copy at each new
+    // best point was a fifth of a trial's instructions).
+    enum : int { kNoBest = 0, kBestStored, kBestAtX, kBestAtTrial };
+    int best_at;
+    // Between the trial phase and the gradient phase of one trip.
+    bool pending = false;
+    double res_kept[NV], ss_kept;
 
     __device__ LaneSolver(const Models<double>* m, const SolverControls& c, const SolveArgs& args)
         : models_(m), ctl(c), a(args) {
-        rec_stride = size_t(gridDim.x) * kLaneBlock * 4;
-        rec_base = static_cast<double*>(a.history) + (size_t(blockIdx.x) * kLaneBlock + threadIdx.x) * 4;
+        rec_base = static_cast<double*>(a.history) + (size_t(blockIdx.x) * lane_records(L) * kLaneBlock + threadIdx.x) * 4;
         if constexpr (BATCH) models_ = static_cast<const Models<double>*>(a.models);
     }
 
     // ------------------------------------------------------------ storage --
-    __device__ __forceinline__ double2* slot(int unit) const {
+    __device__ __forceinline__ static double2* slot(int unit) {
         return reinterpret_cast<double2*>(lane_smem) + unit * kLaneBlock + threadIdx.x;
     }
-    __device__ __forceinline__ void get(int vec, int l, double* v) const {
+    __device__ __forceinline__ static void get(int vec, int l, double* v) {
         const double2* p = slot(vec * 2 * L + 2 * l);
         const double2 u = p[0], w = p[kLaneBlock];
         v[0] = u.x; v[1] = u.y; v[2] = w.x; v[3] = w.y;
     }
-    __device__ __forceinline__ void put(int vec, int l, double v0, double v1, double v2, double v3) const {
+    __device__ __forceinline__ static void put(int vec, int l, double v0, double v1, double v2, double v3) {
         double2* p = slot(vec * 2 * L + 2 * l);
         p[0] = make_double2(v0, v1);
         p[kLaneBlock] = make_double2(v2, v3);
     }
     enum : int { kX = 0, kG = 1, kD = 2 };
-    __device__ __forceinline__ double* rec(int k) const { return rec_base + size_t(k) * rec_stride; }
-    __device__ __forceinline__ double* ring(int s, int w, int l) const { return rec((s * 2 + w) * L + l); }
-    __device__ __forceinline__ double* best_rec(int l) const { return rec(2 * kLaneRing * L + l); }
-    __device__ __forceinline__ double* ox_rec(int l) const { return rec((2 * kLaneRing + 1) * L + l); }
+    // The target colour and the multipliers: in shared memory where it has
+    // room (seven registers pairs more for the loops), else in registers.
+    __device__ __forceinline__ double& extra(int k) const {
+        return reinterpret_cast<double*>(lane_smem + lane_smem_units(L) * kLaneBlock * 16)[k * kLaneBlock + threadIdx.x];
+    }
+    __device__ __forceinline__ double& target(int c) {
+        if constexpr (kSharedTargets) return extra(c); else return target_[c];
+    }
+    __device__ __forceinline__ double& lam(int c) {
+        if constexpr (kSharedTargets) return extra(3 + c); else return lam_[c];
+    }
+    // Record k of a lane whose records start at `base`.
+    __device__ __forceinline__ static double* rec(double* base, int k) { return base + k * (kLaneBlock * 4); }
+    __device__ __forceinline__ static double* ring(double* base, int s, int w, int l) { return rec(base, (s * 2 + w) * L + l); }
+    __device__ __forceinline__ double* ring(int s, int w, int l) const { return ring(rec_base, s, w, l); }
+    __device__ __forceinline__ double* best_rec(int l) const { return rec(rec_base, 2 * kLaneRing * L + l); }
+    __device__ __forceinline__ double* ox_rec(int l) const { return rec(rec_base, (2 * kLaneRing + 1) * L + l); }
+    __device__ __forceinline__ double* residual_rec() const { return rec(rec_base, (2 * kLaneRing + 2) * L); }
+    __device__ __forceinline__ double* outer_rec() const { return rec(rec_base, (2 * kLaneRing + 2) * L + 1); }
 
-    __device__ __forceinline__ void count(int k, uint32_t n = 1) const { if (a.counters) a.counters[5 * size_t(gidx) + k] += n; }
-    __device__ __forceinline__ const double* image() const {
-        if constexpr (BATCH) return a.jobs[job_id].image; else return a.image;
+    // What the method keeps of a pixel between its outer steps.
+    struct Outer {
+        double oldnorm;     // squared residual at the outer step's start
+        int outer, frozen, pixel, gidx, start, job;
+    };
+    __device__ __forceinline__ Outer load_outer() const {
+        double v[4];
+        load_rec(outer_rec(), v);
+        return Outer{v[0], __double2hiint(v[1]), __double2loint(v[1]), __double2hiint(v[2]), __double2loint(v[2]),
+                     __double2hiint(v[3]), __double2loint(v[3])};
     }
-    __device__ __forceinline__ size_t pixels() const {
-        if constexpr (BATCH) return size_t(a.jobs[job_id].n); else return size_t(a.n);
+    __device__ __forceinline__ void store_outer(const Outer& o) const {
+        store_rec(outer_rec(), o.oldnorm, __hiloint2double(o.outer, o.frozen), __hiloint2double(o.pixel, o.gidx),
+                  __hiloint2double(o.start, o.job));
     }
-    __device__ __forceinline__ bool fixed_bounds(int l, int c) const {
-        return l == 0 && (c == 3 ? a.opaque != 0 : (REFINE && a.smooth != 0));
+
+    // Work counters (only when requested).
+    __device__ __forceinline__ void count(int k) const { if (a.counters) ++a.counters[5 * size_t(load_outer().gidx) + k]; }
+    __device__ __forceinline__ static bool fixed_bounds(bool opaque, bool smooth, int l, int c) {
+        return l == 0 && (c == 3 ? opaque : (REFINE && smooth));
     }
-    __device__ __forceinline__ bool fixed_at(int l, int c, double x, double g) const {
-        return fixed_bounds(l, c) || (x <= 0.0 && g > 0.0) || (x >= 1.0 && g < 0.0);
+    __device__ __forceinline__ static bool fixed_at(bool opaque, bool smooth, int l, int c, double x, double g) {
+        return fixed_bounds(opaque, smooth, l, c) || (x <= 0.0 && g > 0.0) || (x >= 1.0 && g < 0.0);
     }
-    __device__ __forceinline__ static double clamp01(double v) { return v < 0.0 ? 0.0 : (v > 1.0 ? 1.0 : v); }
+    // v in [0, 1] (NaN stays NaN), by its bits: the FP64 pipe has the
+    // arithmetic, and its compares are as slow as it is.
+    __device__ __forceinline__ static double clamp01(double v) {
+        const int hi = __double2hiint(v);
+        const bool keep = uint32_t(hi) < 0x3ff00000u || (uint32_t(hi) & 0x7fffffffu) > 0x7ff00000u;
+        return __hiloint2double(keep ? hi : (hi < 0 ? 0 : 0x3ff00000), keep ? __double2loint(v) : 0);
+    }
 
     // The per-channel partial sums, added as the lanes of a group add theirs.
     __device__ __forceinline__ static double sum(const double* v) {
@@ -296,9 +355,9 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         const double n_dd = 1.0 - dd, n_av = 1.0 - av;
         const double ya = __dmul_rn(Y * av, n_dd), zd = __dmul_rn(Z * dd, n_av);
         const double Al = __dadd_rn(zd, mul_add(X * av, dd, ya));
+        const double y = reciprocal(Al);
         double fv[3];
         blend_value3(m.mode[l], t, pc, fv);
-        const double y = __drcp_rn(Al);
         const bool big = Al > 1e-12;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -309,15 +368,24 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         A = Al;
     }
 
-    // Trial point of layer l: x + step d within bounds (the fixed values have
-    // d = 0 and x in [0, 1]), or x itself at the start of an outer step.
-    __device__ __forceinline__ void trial(const double* x, const double* d, bool at_x, double* t) const {
+    // Point of layer l at step s along d, within bounds (the fixed values have
+    // d = 0 and x in [0, 1]; at the start of an outer step d is zero).
+    __device__ __forceinline__ static void point(const double* x, const double* d, double s, double* t) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            if (REFINE && c == 3) { t[c] = x[c]; continue; }
-            const double v = clamp01(mul_add(step, d[c], x[c]));
-            t[c] = at_x ? x[c] : v;
+        for (int c = 0; c < 4; ++c) t[c] = REFINE && c == 3 ? x[c] : clamp01(mul_add(s, d[c], x[c]));
+    }
+
+    // Writes the best point to its records before x or d changes.
+    __device__ __forceinline__ void save_best() {
+        const bool at_x = best_at == kBestAtX;
+#pragma unroll 1
+        for (int l = 0; l < L; ++l) {
+            double x[4], d[4], t[4];
+            get(kX, l, x); get(kD, l, d);
+            point(x, d, best_step, t);
+            store_rec(best_rec(l), at_x ? x[0] : t[0], at_x ? x[1] : t[1], at_x ? x[2] : t[2], at_x ? x[3] : t[3]);
         }
+        best_at = kBestStored;
     }
 
     // Evaluates the objective at the trial point (kLaneTrial) or at x
@@ -329,21 +397,25 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     __device__ __forceinline__ void forward() {
         const Models<double>& m = *models_;
         const bool keep = state == kLaneGrad, at_x = state == kLaneOuter || (keep && !from_trial);
-        bool moved = false;     // some component moved by at least the inner tolerance
+        // (keep) the accepted point is the best point; the best point is lost with x and d.
+        const bool best_here = best_at == kBestAtTrial && best_step == step;
+        const bool best_lost = !at_x && (best_at == kBestAtX || (best_at == kBestAtTrial && !best_here));
+        bool moved = false;     // (keep) some component moved by at least the inner tolerance
         const double tol_lo = ctl.inner_tolerance * (1.0 - 0x1p-48), tol_hi = ctl.inner_tolerance * (1.0 + 0x1p-48);
-        double sl[NV], mo[NV], A = 0.0, pc[3], energy = 0.0, asum = 0.0;
+        double sl[NV], ss[NV], A = 0.0, pc[3], energy = 0.0, asum = 0.0;
+        uint32_t largest = 0;   // high word of the largest motion of a component
 #pragma unroll
-        for (int c = 0; c < NV; ++c) { sl[c] = 0.0; mo[c] = 0.0; }
+        for (int c = 0; c < NV; ++c) { sl[c] = 0.0; ss[c] = 0.0; }
 #pragma unroll 1
         for (int l = 0; l < L; ++l) {
-            double x[4], d[4], g[4], t[4];
+            double x[4], d[4], g[4], t[4], s[4] = {0.0, 0.0, 0.0, 0.0};
             get(kX, l, x); get(kD, l, d); get(kG, l, g);
-            trial(x, d, at_x, t);
+            point(x, d, step, t);
 #pragma unroll
             for (int c = 0; c < NV; ++c) {
-                const double delta = t[c] - x[c];
-                sl[c] = mul_add(g[c], delta, sl[c]);
-                mo[c] = mul_add(delta, delta, mo[c]);
+                s[c] = t[c] - x[c];
+                sl[c] = mul_add(g[c], s[c], sl[c]);
+                largest = max(largest, uint32_t(__double2hiint(s[c])) & 0x7fffffffu);
             }
             const double av = t[3];
             const double d0 = t[0] - m.mean[l][0], d1 = t[1] - m.mean[l][1], d2 = t[2] - m.mean[l][2];
@@ -356,53 +428,57 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
             asum += av;
             compose(m, l, t, av, A, pc);
             if (keep) {
-                if (!at_x) {
-                    double s[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-                    for (int c = 0; c < NV; ++c) {
-                        s[c] = t[c] - x[c];
-                        // |s| / (1 + |x|) against the tolerance without the
-                        // division, except where rounding could decide.
-                        const double w = 1.0 + fabs(x[c]), as = fabs(s[c]);
-                        if (!(as < tol_lo * w)) moved = moved || as > tol_hi * w || step_reaches(as, w, ctl.inner_tolerance);
-                    }
-                    store_rec(ring(next, 0, l), s[0], s[1], s[2], s[3]);
-                    put(kX, l, t[0], t[1], t[2], t[3]);
+                for (int c = 0; c < NV; ++c) {
+                    ss[c] = mul_add(s[c], s[c], ss[c]);
+                    // |s| / (1 + |x|) against the tolerance without the
+                    // division, except where rounding could decide.
+                    const double w = 1.0 + fabs(x[c]), as = fabs(s[c]);
+                    if (!(as < tol_lo * w)) moved = moved || as > tol_hi * w || step_reaches(as, w, ctl.inner_tolerance);
                 }
+                if (best_lost) {
+                    double b[4];
+                    point(x, d, best_at == kBestAtX ? 0.0 : best_step, b);
+                    store_rec(best_rec(l), b[0], b[1], b[2], b[3]);
+                }
+                store_rec(ring(next, 0, l), s[0], s[1], s[2], s[3]);
+                put(kX, l, t[0], t[1], t[2], t[3]);
                 put(kD, l, pc[0], pc[1], pc[2], A);
             }
         }
+        double res[NV];
+#pragma unroll
+        for (int c = 0; c < NV; ++c) res[c] = c < 3 ? pc[c < 3 ? c : 0] - target(c < 3 ? c : 0) : A - 1.0;
         if (keep) {
             small_change = small_change || !moved;
-            ss_kept = sum(mo);
+            if (best_here) best_at = kBestAtX;
+            if (best_lost) best_at = kBestStored;
+            ss_kept = sum(ss);
+#pragma unroll
+            for (int c = 0; c < NV; ++c) res_kept[c] = res[c];
+            store_rec(residual_rec(), res[0], res[1], res[2], res[NV - 1]);
             return;
         }
         if (!REFINE) energy += 0.01 * asum;
-        double res[NV], terms[NV], nn[NV];
+        double terms[NV], nn[NV];
 #pragma unroll
         for (int c = 0; c < NV; ++c) {
-            res[c] = c < 3 ? pc[c < 3 ? c : 0] - target[c < 3 ? c : 0] : A - 1.0;
-            terms[c] = mul_add(0.5 * rho * res[c], res[c], -(lam[c] * res[c]));
+            terms[c] = mul_add(0.5 * rho * res[c], res[c], -(lam(c) * res[c]));
             nn[c] = res[c] * res[c];
         }
-        const double norm = sum(nn), value = energy + sum(terms);
-        const double slope = sum(sl), motion = sum(mo);
+        const double norm = sum(nn), value = energy + sum(terms), slope = sum(sl);
 
-        // A trial that does not move ends the attempt, unevaluated.
-        if (!at_x && motion == 0.0) { attempt_failed(); return; }
+        // A trial that does not move (whose sum of squared motions is zero:
+        // squares below 2^-1074) ends the attempt, unevaluated.
+        if (!at_x && largest < 0x1e600000u) { attempt_failed(); return; }
         const double tol2 = ctl.outer_tolerance * ctl.outer_tolerance;
         const bool feasible = norm < tol2;
         if (isfinite(energy) && isfinite(norm) &&
-            (!have_best || (feasible && (best_norm >= tol2 || energy < best_energy)) ||
+            (best_at == kNoBest || (feasible && (best_norm >= tol2 || energy < best_energy)) ||
              (!feasible && best_norm >= tol2 && norm < best_norm))) {
-            have_best = true; best_norm = norm; best_energy = energy; best_moved = true;
-#pragma unroll 1
-            for (int l = 0; l < L; ++l) {
-                double x[4], d[4], t[4];
-                get(kX, l, x); get(kD, l, d);
-                trial(x, d, at_x, t);
-                store_rec(best_rec(l), t[0], t[1], t[2], t[3]);
-            }
+            best_norm = norm; best_energy = energy; best_moved = true;
+            best_at = at_x ? kBestAtX : kBestAtTrial;
+            best_step = step;
         }
         // Evaluations are counted as the method makes them: a first trial
         // with its gradient, and a later trial that is accepted once more,
@@ -412,7 +488,7 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         if (counted_grad) { count(1); ++n_grad; }
         if (at_x) {
             f = value;
-            oldnorm = norm;
+            outer_rec()[0] = norm;
             valid = 0; next = 0; it = 0;
             from_trial = false;
             state = kLaneGrad;
@@ -428,11 +504,8 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
             } else {
                 step *= 0.5;
                 if (++bt >= 32) attempt_failed();
-                return;
             }
         }
-#pragma unroll
-        for (int c = 0; c < NV; ++c) resx[c] = res[c];
     }
 
     __device__ __noinline__ static bool step_reaches(double as, double w, double tol) { return !(as / w < tol); }
@@ -451,9 +524,9 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         const Models<double>& m = *models_;
         const bool at_x = !from_trial;
         // Reverse sweep; layer l's slot of d turns from its composite into its gradient.
-        double adj[3], adj3 = REFINE ? 0.0 : rho * resx[NV - 1] - lam[NV - 1];
+        double adj[3], adj3 = REFINE ? 0.0 : rho * res_kept[NV - 1] - lam(NV - 1);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) adj[c] = rho * resx[c] - lam[c];
+        for (int c = 0; c < 3; ++c) adj[c] = rho * res_kept[c] - lam(c);
 #pragma unroll 1
         for (int l = L - 1; l >= 0; --l) {
             double t[4], ng[4];
@@ -483,7 +556,7 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
                 const bool big = Al > 1e-12;
                 double fv[3], fs[3], fd[3], ga[3], gp[3];
                 blend_all3(m.mode[l], t, q, fv, fs, fd);
-                const double y = __drcp_rn(Al);
+                const double y = reciprocal(Al);
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     const double v = adj[c], s = t[c], cc = q[c];
@@ -518,7 +591,7 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
             put(kD, l, ng[0], ng[1], ng[2], ng[3]);
         }
         if (at_x) {
-#pragma unroll 1
+#pragma unroll
             for (int l = 0; l < L; ++l) {
                 double ng[4];
                 get(kD, l, ng);
@@ -530,10 +603,13 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         double sy[NV], yy[NV], ya = 0.0;
 #pragma unroll
         for (int c = 0; c < NV; ++c) { sy[c] = 0.0; yy[c] = 0.0; }
-#pragma unroll 1
+        double step_taken[L][4];
+#pragma unroll
+        for (int l = 0; l < L; ++l) load_rec(ring(next, 0, l), step_taken[l]);
+#pragma unroll
         for (int l = 0; l < L; ++l) {
-            double ng[4], g[4], s[4], yv[4] = {0.0, 0.0, 0.0, 0.0};
-            load_rec(ring(next, 0, l), s);
+            double ng[4], g[4], yv[4] = {0.0, 0.0, 0.0, 0.0};
+            const double* s = step_taken[l];
             get(kD, l, ng); get(kG, l, g);
 #pragma unroll
             for (int c = 0; c < NV; ++c) {
@@ -573,6 +649,23 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     // direction) or the steepest-descent attempt (kLaneSteep).
     __device__ __forceinline__ void direction() {
         const bool steep = state == kLaneSteep;
+        if (!steep) count(2);
+        if (best_at == kBestAtTrial) save_best();
+        const int what = form_direction(rec_base, valid, next, steep, a.opaque != 0, a.smooth != 0, isfinite(f));
+        if (what == kStationary) { state = kLaneEnd; return; }
+        if (what == kReset) { valid = 0; next = 0; }
+        second = steep;
+        bt = 0;
+        step = 1.0;
+        state = kLaneTrial;
+    }
+
+    // Forms d from x, g and the ring. Out of line, so that the unrolled loops
+    // have the registers to themselves (the caller's state goes to the stack
+    // once per call).
+    enum : int { kStationary = 0, kFormed = 1, kReset = 2 };
+    __device__ __noinline__ static int form_direction(double* base, int valid, int next, bool steep, bool opaque,
+                                                      bool smooth, bool finite_f) {
         uint32_t freem = 0;
         {
             double pg[NV];
@@ -585,21 +678,22 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
                 v[3] = 0.0;
 #pragma unroll
                 for (int c = 0; c < NV; ++c) {
-                    const bool fr = !fixed_at(l, c, x[c], g[c]);
+                    const bool fr = !fixed_at(opaque, smooth, l, c, x[c], g[c]);
                     freem |= fr ? 1u << (l * 4 + c) : 0u;
                     v[c] = fr ? g[c] : 0.0;
                     pg[c] = mul_add(v[c], v[c], pg[c]);
                 }
                 put(kD, l, v[0], v[1], v[2], v[3]);
             }
-            if (!steep) {
-                count(2);
-                if (sum(pg) < 1e-16 || !isfinite(f)) { state = kLaneEnd; return; }
-            }
+            if (!steep && (sum(pg) < 1e-16 || !finite_f)) return kStationary;
         }
         double q[L][4];
 #pragma unroll
         for (int l = 0; l < L; ++l) get(kD, l, q[l]);
+        // The pairs' components outside the free set are read as zeros (a
+        // select each; skipping their operations instead takes a branch each,
+        // and the kernel 1.1 times as long). q is zero there throughout, so
+        // its own products need no select.
         double scaling = 1.0;
         bool have_scaling = false;
         double2* coeff = slot(4 * L);
@@ -610,30 +704,32 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
             double dot[NV], sy[NV], ss[NV], yy[NV];
 #pragma unroll
             for (int c = 0; c < NV; ++c) { dot[c] = 0.0; sy[c] = 0.0; ss[c] = 0.0; yy[c] = 0.0; }
+            double ym[L][4];
+#pragma unroll
+            for (int l = 0; l < L; ++l) load_rec(ring(base, k, 1, l), ym[l]);
 #pragma unroll
             for (int l = 0; l < L; ++l) {
-                double sv[4], yv[4];
-                load_rec(ring(k, 0, l), sv); load_rec(ring(k, 1, l), yv);
+                double sv[4];
+                double* yv = ym[l];
+                load_rec(ring(base, k, 0, l), sv);
 #pragma unroll
-                for (int c = 0; c < NV; ++c)
-                    if (freem >> (l * 4 + c) & 1u) {
-                        dot[c] = mul_add(sv[c], q[l][c], dot[c]);
-                        sy[c] = mul_add(sv[c], yv[c], sy[c]);
-                        ss[c] = mul_add(sv[c], sv[c], ss[c]);
-                        yy[c] = mul_add(yv[c], yv[c], yy[c]);
-                    }
+                for (int c = 0; c < NV; ++c) {
+                    const bool fr = freem >> (l * 4 + c) & 1u;
+                    const double s1 = fr ? sv[c] : 0.0, y1 = fr ? yv[c] : 0.0;
+                    yv[c] = y1;
+                    dot[c] = mul_add(s1, q[l][c], dot[c]);
+                    sy[c] = mul_add(s1, y1, sy[c]);
+                    ss[c] = mul_add(s1, s1, ss[c]);
+                    yy[c] = mul_add(y1, y1, yy[c]);
+                }
             }
             const double syt = sum(sy), yyt = sum(yy);
             const double inv = curvature(syt, sum(ss), yyt) ? __drcp_rn(syt) : 0.0;
             const double co = sum(dot) * inv;
 #pragma unroll
-            for (int l = 0; l < L; ++l) {
-                double yv[4];
-                load_rec(ring(k, 1, l), yv);
+            for (int l = 0; l < L; ++l)
 #pragma unroll
-                for (int c = 0; c < NV; ++c)
-                    if (freem >> (l * 4 + c) & 1u) q[l][c] = mul_add(-co, yv[c], q[l][c]);
-            }
+                for (int c = 0; c < NV; ++c) q[l][c] = mul_add(-co, ym[l][c], q[l][c]);
             if (!have_scaling && inv > 0.0 && yyt > 0.0) { scaling = syt / yyt; have_scaling = true; }
             coeff[j * kLaneBlock] = make_double2(co, inv);
         }
@@ -646,27 +742,23 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         for (int j = valid - 1; j >= 0; --j) {
             int k = next - 1 - j;
             k = k < 0 ? k + kLaneRing : k;
-            double dot[NV];
+            double dot[NV], sv[L][4];
 #pragma unroll
             for (int c = 0; c < NV; ++c) dot[c] = 0.0;
 #pragma unroll
             for (int l = 0; l < L; ++l) {
                 double yv[4];
-                load_rec(ring(k, 1, l), yv);
+                load_rec(ring(base, k, 1, l), yv); load_rec(ring(base, k, 0, l), sv[l]);
 #pragma unroll
-                for (int c = 0; c < NV; ++c)
-                    if (freem >> (l * 4 + c) & 1u) dot[c] = mul_add(yv[c], q[l][c], dot[c]);
+                for (int c = 0; c < NV; ++c) dot[c] = mul_add(yv[c], q[l][c], dot[c]);
             }
             const double2 ci = coeff[j * kLaneBlock];
             const double w = mul_add(-sum(dot), ci.y, ci.x);
 #pragma unroll
-            for (int l = 0; l < L; ++l) {
-                double sv[4];
-                load_rec(ring(k, 0, l), sv);
+            for (int l = 0; l < L; ++l)
 #pragma unroll
                 for (int c = 0; c < NV; ++c)
-                    if (freem >> (l * 4 + c) & 1u) q[l][c] = mul_add(w, sv[c], q[l][c]);
-            }
+                    q[l][c] = mul_add(w, freem >> (l * 4 + c) & 1u ? sv[l][c] : 0.0, q[l][c]);
         }
 #pragma unroll
         for (int l = 0; l < L; ++l) put(kD, l, q[l][0], q[l][1], q[l][2], q[l][3]);
@@ -680,89 +772,104 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
 #pragma unroll
             for (int c = 0; c < NV; ++c) {
                 double v = -d[c];
-                if (fixed_bounds(l, c) || (x[c] <= 0.0 && v < 0.0) || (x[c] >= 1.0 && v > 0.0)) v = 0.0;
+                if (fixed_bounds(opaque, smooth, l, c) || (x[c] <= 0.0 && v < 0.0) || (x[c] >= 1.0 && v > 0.0)) v = 0.0;
                 d[c] = v;
                 descent[c] = mul_add(v, g[c], descent[c]);
             }
             put(kD, l, d[0], d[1], d[2], d[3]);
         }
         if (!steep && !(sum(descent) < 0.0)) {
-            valid = 0; next = 0;
 #pragma unroll 1
             for (int l = 0; l < L; ++l) {
                 double x[4], g[4], d[4];
                 get(kX, l, x); get(kG, l, g);
                 d[3] = 0.0;
 #pragma unroll
-                for (int c = 0; c < NV; ++c) d[c] = fixed_at(l, c, x[c], g[c]) ? 0.0 : -g[c];
+                for (int c = 0; c < NV; ++c) d[c] = fixed_at(opaque, smooth, l, c, x[c], g[c]) ? 0.0 : -g[c];
                 put(kD, l, d[0], d[1], d[2], d[3]);
             }
+            return kReset;
         }
-        second = steep;
-        bt = 0;
-        step = 1.0;
-        state = kLaneTrial;
+        return kFormed;
     }
 
     // -------------------------------------------------------- outer steps --
     // End of an outer step (kLaneEnd): multipliers, penalty, and the next
-    // outer step (true), or the next start / the pixel's result.
+    // outer step, the next start, or the pixel's result.
     enum : int { kNextOuter, kNextStart, kFinished };
-    __device__ __forceinline__ int end_outer() {
-        const double tol2 = ctl.outer_tolerance * ctl.outer_tolerance;
-        double nn[NV], mo[NV];
+    __device__ __forceinline__ int end_outer(Outer& o) {
+        double r[4], ox[L][4], nn[NV], mo[NV];
+        o = load_outer();
+        load_rec(residual_rec(), r);
 #pragma unroll
-        for (int c = 0; c < NV; ++c) { nn[c] = resx[c] * resx[c]; mo[c] = 0.0; }
+        for (int l = 0; l < L; ++l) load_rec(ox_rec(l), ox[l]);
+        const double tol2 = ctl.outer_tolerance * ctl.outer_tolerance;
+#pragma unroll
+        for (int c = 0; c < NV; ++c) { nn[c] = r[c] * r[c]; mo[c] = 0.0; }
         const double norm = sum(nn);
         const bool feasible = norm < tol2;
 #pragma unroll
-        for (int c = 0; c < NV; ++c) lam[c] = mul_add(-rho, resx[c], lam[c]);
-        if (norm > 0.0625 * oldnorm) rho *= 10.0;
-#pragma unroll 1
+        for (int c = 0; c < NV; ++c) lam(c) = mul_add(-rho, r[c], lam(c));
+        if (norm > 0.0625 * o.oldnorm) rho *= 10.0;
+#pragma unroll
         for (int l = 0; l < L; ++l) {
-            double x[4], o[4];
-            load_rec(ox_rec(l), o);
+            double x[4];
             get(kX, l, x);
 #pragma unroll
-            for (int c = 0; c < NV; ++c) { const double dl = x[c] - o[c]; mo[c] = mul_add(dl, dl, mo[c]); }
+            for (int c = 0; c < NV; ++c) { const double dl = x[c] - ox[l][c]; mo[c] = mul_add(dl, dl, mo[c]); }
         }
         const double motion = sum(mo);
-        frozen = (motion == 0.0 && !best_moved) ? frozen + 1 : 0;
-        if (ctl.frozen_stop > 0 && frozen >= ctl.frozen_stop) {
-            if (start + 1 < ctl.starts) { ++start; return kNextStart; }
-            return kFinished;
+        o.frozen = (motion == 0.0 && !best_moved) ? o.frozen + 1 : 0;
+        int what = kFinished;
+        if (!(ctl.frozen_stop > 0 && o.frozen >= ctl.frozen_stop) && !(motion < tol2 && feasible) &&
+            o.outer + 1 < ctl.outer) {
+            ++o.outer;
+            what = kNextOuter;
+        } else if (o.start + 1 < ctl.starts) {
+            ++o.start;
+            what = kNextStart;
         }
-        if (!(motion < tol2 && feasible) && outer + 1 < ctl.outer) { ++outer; return kNextOuter; }
-        if (start + 1 < ctl.starts) { ++start; return kNextStart; }
-        return kFinished;
+        if (best_at == kBestAtTrial || (best_at == kBestAtX && what == kNextStart)) save_best();
+        return what;
     }
 
-    __device__ __forceinline__ void begin_outer() {
+    __device__ __forceinline__ void begin_outer(const Outer& o) {
+        store_outer(o);
         count(4);
-#pragma unroll 1
+#pragma unroll
         for (int l = 0; l < L; ++l) {
             double x[4];
             get(kX, l, x);
             store_rec(ox_rec(l), x[0], x[1], x[2], x[3]);
+            put(kD, l, 0.0, 0.0, 0.0, 0.0);
         }
         best_moved = false;
+        step = 0.0;
         state = kLaneOuter;
     }
 
-    __device__ __forceinline__ double pinned_alpha(int l) const {
-        return (a.opaque && l == 0) ? 1.0 : a.targets[size_t(l) * size_t(a.n) + pixel];
+    __device__ __forceinline__ const double* image(const Outer& o) const {
+        if constexpr (BATCH) return a.jobs[o.job].image; else return a.image;
     }
-    __device__ __forceinline__ double background(int c) const { return a.targets[(size_t(L) + c) * size_t(a.n) + pixel]; }
+    __device__ __forceinline__ size_t pixels(const Outer& o) const {
+        if constexpr (BATCH) return size_t(a.jobs[o.job].n); else return size_t(a.n);
+    }
+    __device__ __forceinline__ double pinned_alpha(const Outer& o, int l) const {
+        return (a.opaque && l == 0) ? 1.0 : a.targets[size_t(l) * size_t(a.n) + o.pixel];
+    }
+    __device__ __forceinline__ double background(const Outer& o, int c) const {
+        return a.targets[(size_t(L) + c) * size_t(a.n) + o.pixel];
+    }
 
     // The start-0 seed of component c of layer l.
-    __device__ __forceinline__ double seed(int l, int c) const {
-        const size_t i = size_t(pixel);
+    __device__ __forceinline__ double seed(const Outer& o, int l, int c) const {
+        const size_t i = size_t(o.pixel);
         if constexpr (REFINE) {
-            if (c == 3) return pinned_alpha(l);
-            return (a.smooth && l == 0) ? background(c) : a.first[(size_t(l) * size_t(a.n) + i) * 4 + c];
+            if (c == 3) return pinned_alpha(o, l);
+            return (a.smooth && l == 0) ? background(o, c) : a.first[(size_t(l) * size_t(a.n) + i) * 4 + c];
         } else {
             const float* wp;
-            if constexpr (BATCH) wp = a.jobs[job_id].warm; else wp = a.warm;
+            if constexpr (BATCH) wp = a.jobs[o.job].warm; else wp = a.warm;
             if (wp) return double(wp[i * size_t(4 * L) + (c == 3 ? l : L + 3 * l + c)]);
             if (c == 3) return (a.opaque && l == 0) ? 1.0 : 0.5;
             return fmin(1.0, fmax(0.0, models_->mean[l][c]));
@@ -770,62 +877,77 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     }
 
     // Bounds of component c of layer l applied to v.
-    __device__ __forceinline__ double clamp_bounds(int l, int c, double v) const {
+    __device__ __forceinline__ double clamp_bounds(const Outer& o, int l, int c, double v) const {
         if (REFINE && c == 3) return v;
         double lo = 0.0, hi = 1.0;
         if (l == 0 && c == 3 && a.opaque) lo = 1.0;
-        if (REFINE && l == 0 && c != 3 && a.smooth) lo = hi = background(c);
+        if (REFINE && l == 0 && c != 3 && a.smooth) lo = hi = background(o, c);
         return v < lo ? lo : (v > hi ? hi : v);
     }
 
     // Component c of layer l of x in shared memory.
-    __device__ __forceinline__ double* x_at(int l, int c) const {
+    __device__ __forceinline__ static double* x_at(int l, int c) {
         return reinterpret_cast<double*>(slot(kX * 2 * L + 2 * l + (c >> 1))) + (c & 1);
     }
 
-    // Starting point `start` (one component at a time: rare, so kept small).
-    __device__ __forceinline__ void begin_start() {
+    // Starting point o.start: the seeds, all loads in flight at once; the
+    // further starts one component at a time (rare).
+    __device__ __forceinline__ void begin_start(Outer& o) {
+        if (o.start == 0) {
+            double v[L][4];
+#pragma unroll
+            for (int l = 0; l < L; ++l)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) v[l][c] = seed(o, l, c);
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (!(REFINE && l == 0 && c != 3 && a.smooth)) v[l][c] = clamp_bounds(o, l, c, v[l][c]);
+                put(kX, l, v[l][0], v[l][1], v[l][2], v[l][3]);
+            }
+        } else {
+            further_start(o);
+        }
+#pragma unroll
+        for (int c = 0; c < NV; ++c) lam(c) = 0.0;
+        rho = 100.0;
+        o.outer = 0;
+        o.frozen = 0;
+    }
+
+    __device__ __forceinline__ void further_start(const Outer& o) const {
         const Models<double>& m = *models_;
-        const int s = start;
+        const int s = o.start;
 #pragma unroll 1
         for (int k = 0; k < 4 * L; ++k) {
             const int l = k >> 2, c = k & 3;
-            double v = seed(l, c);
-            if (s == 1) {
-                if (c != 3) v = (!REFINE && l == 0) ? fmin(1.0, fmax(0.0, image()[3 * size_t(pixel) + c])) : m.mean[l][c];
-                else if (!REFINE) v = l == 0 ? 1.0 : 0.0;
-            } else if (s == 2) {
-                if (c != 3) v = fmax(0.05, fmin(0.95, m.mean[l][c]));
-                else if (!REFINE) v = 0.5;
-            }
-            *x_at(l, c) = clamp_bounds(l, c, v);
+            double v;
+            if (c == 3) v = REFINE ? pinned_alpha(o, l) : (s == 1 ? (l == 0 ? 1.0 : 0.0) : 0.5);
+            else if (s == 2) v = fmax(0.05, fmin(0.95, m.mean[l][c]));
+            else v = (!REFINE && l == 0) ? fmin(1.0, fmax(0.0, image(o)[3 * size_t(o.pixel) + c])) : m.mean[l][c];
+            *x_at(l, c) = clamp_bounds(o, l, c, v);
         }
-        if (s == 2) {
-            // Move Dodge/Burn sources into the unsaturated branch.
+        if (s != 2) return;
+        // Move Dodge/Burn sources into the unsaturated branch.
 #pragma unroll 1
-            for (int c = 0; c < 3; ++c) {
-                double da = *x_at(0, 3), dest = *x_at(0, c);
+        for (int c = 0; c < 3; ++c) {
+            double da = *x_at(0, 3), dest = *x_at(0, c);
 #pragma unroll 1
-                for (int l = 1; l < L; ++l) {
-                    const double al = *x_at(l, 3), X = m.fX[l], Y = m.fY[l], Z = m.fZ[l];
-                    const double Al = X * al * da + Y * al * (1.0 - da) + Z * da * (1.0 - al);
-                    double sv = *x_at(l, c);
-                    if (dest >= 0.0 && dest <= 1.0 && m.mode[l] == 6) sv = fmin(sv, fmax(0.0, 1.0 - dest - 0.05));
-                    if (dest >= 0.0 && dest <= 1.0 && m.mode[l] == 7) sv = fmax(sv, fmin(1.0, 1.0 - dest + 0.05));
-                    sv = clamp_bounds(l, c, sv);
-                    *x_at(l, c) = sv;
-                    const double pre = blend_value_call<double>(m.mode[l], sv, dest) * al * da +
-                                       Y * al * (1.0 - da) * sv + Z * da * (1.0 - al) * dest;
-                    dest = Al > 1e-12 ? pre / Al : pre;
-                    da = Al;
-                }
+            for (int l = 1; l < L; ++l) {
+                const double al = *x_at(l, 3), X = m.fX[l], Y = m.fY[l], Z = m.fZ[l];
+                const double Al = X * al * da + Y * al * (1.0 - da) + Z * da * (1.0 - al);
+                double sv = *x_at(l, c);
+                if (dest >= 0.0 && dest <= 1.0 && m.mode[l] == 6) sv = fmin(sv, fmax(0.0, 1.0 - dest - 0.05));
+                if (dest >= 0.0 && dest <= 1.0 && m.mode[l] == 7) sv = fmax(sv, fmin(1.0, 1.0 - dest + 0.05));
+                sv = clamp_bounds(o, l, c, sv);
+                *x_at(l, c) = sv;
+                const double pre = blend_value_call<double>(m.mode[l], sv, dest) * al * da +
+                                   Y * al * (1.0 - da) * sv + Z * da * (1.0 - al) * dest;
+                dest = Al > 1e-12 ? pre / Al : pre;
+                da = Al;
             }
         }
-#pragma unroll
-        for (int c = 0; c < NV; ++c) lam[c] = 0.0;
-        rho = 100.0;
-        outer = 0;
-        frozen = 0;
     }
 
     // ------------------------------------------------------------- pixels --
@@ -833,30 +955,46 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     // list. The point written is the best point, whose constraint norm is
     // best_norm (the same operations on the same values as a check of the
     // written point); a pixel without one writes its seed, checked here.
-    __device__ __forceinline__ void store(bool skipped) {
-        const size_t n = pixels(), i = size_t(pixel);
+    __device__ __forceinline__ void store(const Outer& o, bool skipped) {
+        const size_t n = pixels(o), i = size_t(o.pixel);
         double* outp;
         int32_t* stp;
-        if constexpr (BATCH) { outp = a.jobs[job_id].out; stp = a.jobs[job_id].status; }
+        if constexpr (BATCH) { outp = a.jobs[o.job].out; stp = a.jobs[o.job].status; }
         else { outp = a.out; stp = a.status; }
-#pragma unroll 1
-        for (int k = 0; k < 4 * L; ++k) {
-            const int l = k >> 2, c = k & 3;
-            double v = have_best ? best_rec(l)[c] : seed(l, c);
-            if (REFINE && c == 3) v = pinned_alpha(l);
-            if (REFINE && c != 3 && l == 0 && a.smooth) v = background(c);
-            if (!REFINE && c == 3 && l == 0 && a.opaque) v = 1.0;
-            outp[(size_t(l) * n + i) * 4 + c] = v;
+        double v[L][4];
+        if (best_at == kBestStored) {
+#pragma unroll
+            for (int l = 0; l < L; ++l) load_rec(best_rec(l), v[l]);
+        } else if (best_at == kBestAtX) {
+#pragma unroll
+            for (int l = 0; l < L; ++l) get(kX, l, v[l]);
+        } else {
+#pragma unroll
+            for (int l = 0; l < L; ++l)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) v[l][c] = seed(o, l, c);
         }
+#pragma unroll
+        for (int l = 0; l < L; ++l) {
+            if (REFINE) v[l][3] = pinned_alpha(o, l);
+            else if (l == 0 && a.opaque) v[l][3] = 1.0;
+            if (REFINE && l == 0 && a.smooth)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) v[l][c] = background(o, c);
+        }
+#pragma unroll
+        for (int l = 0; l < L; ++l)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) outp[(size_t(l) * n + i) * 4 + c] = v[l][c];   // (8-byte aligned, as the caller's buffer)
         if (skipped) {
             if (stp) stp[i] = 8;
             if (a.input_failed) atomicAdd(a.input_failed, 1);
             return;
         }
-        if (!have_best) best_norm = written_norm(*models_, outp, image() + 3 * i, n, i);
+        if (best_at == kNoBest) best_norm = written_norm(*models_, outp, image(o) + 3 * i, n, i);
         const bool miss = !(best_norm < ctl.outer_tolerance * ctl.outer_tolerance);
         if (stp) stp[i] = miss ? 3 : 0;
-        if (miss && a.miss_list) a.miss_list[atomicAdd(a.miss_count, 1)] = int32_t(gidx);
+        if (miss && a.miss_list) a.miss_list[atomicAdd(a.miss_count, 1)] = int32_t(o.gidx);
     }
 
     // Constraint norm of the written point, one channel at a time.
@@ -889,29 +1027,31 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
 
     // Loads the pixel of queue entry `job`; false when it is written without
     // a solve (refinement targets that cannot be normalized).
-    __device__ __forceinline__ bool load(int job) {
-        gidx = a.list ? a.list[job] : (a.order ? a.order[job] : a.first_pixel + job);
-        int i = gidx;
+    __device__ __forceinline__ bool load(Outer& o, int job) {
+        o.gidx = a.list ? a.list[job] : (a.order ? a.order[job] : a.first_pixel + job);
+        o.pixel = o.gidx;
+        o.job = 0;
         if constexpr (BATCH) {
             int lo = 0, hi = a.job_count - 1;
             while (lo < hi) {
                 const int mid = (lo + hi + 1) >> 1;
-                if (a.jobs[mid].offset <= int64_t(gidx)) lo = mid; else hi = mid - 1;
+                if (a.jobs[mid].offset <= int64_t(o.gidx)) lo = mid; else hi = mid - 1;
             }
-            job_id = lo;
+            o.job = lo;
             models_ = static_cast<const Models<double>*>(a.models) + a.jobs[lo].model;
-            i = gidx - int(a.jobs[lo].offset);
+            o.pixel = o.gidx - int(a.jobs[lo].offset);
         }
-        pixel = i;
-        const double* p = image() + 3 * size_t(i);
+        const size_t i = size_t(o.pixel);
+        const double* p = image(o) + 3 * i;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) target[c] = p[c];
-        have_best = false;
+        for (int c = 0; c < 3; ++c) target(c) = p[c];
+        best_at = kNoBest;
         best_norm = INFINITY; best_energy = INFINITY;
         if (a.counters)
 #pragma unroll
-            for (int k = 0; k < 5; ++k) a.counters[5 * size_t(gidx) + k] = 0;
-        start = 0;
+            for (int k = 0; k < 5; ++k) a.counters[5 * size_t(o.gidx) + k] = 0;
+        o.start = 0;
+        o.oldnorm = 0.0;
         return !(REFINE && a.input_status && a.input_status[i] != 0);
     }
 
@@ -930,14 +1070,15 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
             if (ne > 0 && (8 * ne >= kOuterQuorum * live || nf == 0)) {
                 int what = kFinished;
                 bool write = false, skipped = false;
+                Outer o{};
                 if (state == kLaneEnd) {
-                    what = end_outer();
+                    what = end_outer(o);
                     write = what == kFinished;
                 }
                 // Finished pixels are written, and the lanes without a pixel
                 // take the next queue entries together.
                 for (;;) {
-                    if (write) { store(skipped); write = false; state = kLaneFetch; }
+                    if (write) { store(o, skipped); write = false; state = kLaneFetch; }
                     const unsigned want = __ballot_sync(full, state == kLaneFetch);
                     if (want == 0) break;
                     const int leader = __ffs(want) - 1;
@@ -950,13 +1091,13 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
                         else {
                             state = kLaneEnd;
                             what = kNextStart;
-                            if (!load(job)) write = skipped = true;
+                            if (!load(o, job)) write = skipped = true;
                         }
                     }
                 }
                 if (state == kLaneEnd) {
-                    if (what == kNextStart) begin_start();
-                    begin_outer();
+                    if (what == kNextStart) begin_start(o);
+                    begin_outer(o);
                 }
             }
             __syncwarp();

@@ -30,4 +30,16 @@ UNB_HOST_DEVICE double quotient(double a, double b, double y) {
     return fma(r, y, q);
 }
 
+// RN(1/b) from an approximation y of relative error below 2^-16, for b and
+// 1/b well inside the exponent range: Newton's iteration with fused residuals
+// (Markstein, as above). The last step rounds correctly from a reciprocal
+// within one unit in the last place, except where b's significand is all
+// ones: the result there is the number above a power of two, and the
+// iteration ends on either of the two.
+UNB_HOST_DEVICE double refine_reciprocal(double b, double y) {
+    y = fma(y, fma(-b, y, 1.0), y);
+    y = fma(y, fma(-b, y, 1.0), y);
+    return fma(y, fma(-b, y, 1.0), y);
+}
+
 }  // namespace unb

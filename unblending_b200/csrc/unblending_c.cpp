@@ -452,18 +452,16 @@ int fp64_variant(const unblending_solver_options& so, bool refine) {
     return so.fp64_variant >= 0 ? so.fp64_variant : default_fp64_variant(refine);
 }
 
-// Whether an FP64 solve of up to `count` pixels runs one pixel per lane
-// (lane_solver.cuh) rather than on quads: by default, unless the caller names
-// a quad variant or a block size. A first pass of up to three layers and fewer
-// than 32,768 pixels stays on quads: there the last pixels' serial chain
-// decides, and a quad's evaluation is the shorter one (three layers, first
-// pass, lanes / quads in ms: 5,184 pixels 2.4 / 2.0, 16,384 2.4 / 1.9, 30,976
-// 3.0 / 2.6, 65,536 3.3 / 4.0; refinement 2.5 / 3.0, 2.8 / 3.4, 2.8 / 3.1, 3.2 /
-// 4.5; five layers, first pass: 576 pixels 3.2 / 4.8, 16,384 5.3 / 5.6, 65,536
-// 7.2 / 12.7; eight layers, 576 4.2 / 9.1, 65,536 14 / 57).
-bool lane_solve(const unblending_solver_options& so, int L, bool refine, int64_t count) {
-    return so.fp64_variant < 0 && so.threads_per_block == 0 && (refine || L > 3 || count >= 32768);
-}
+// Whether an FP64 solve runs one pixel per lane (lane_solver.cuh) rather than
+// on quads: unless the caller names a quad variant or a block size. Lanes are
+// the faster at every size, by the length of the last pixels' serial chains in
+// the smallest launches (a launch spreads its pixels over all warps) and by
+// throughput in the large ones. Lanes / quads, ms, first pass and refinement:
+// three layers, 64 pixels 0.6 / 0.8 and 0.3 / 0.7, 5,184 1.7 / 2.1 and 1.5 / 3.0,
+// 65,536 2.3 / 4.1 and 2.0 / 4.6; five layers, 576 2.7 / 4.6 and 2.0 / 6.5, 65,536
+// 6.2 / 12.8 and 4.6 / 12.5; eight layers, 576 3.6 / 9.2 and 3.0 / 9.2, 65,536 11 / 57
+// and 8.7 / 28.
+bool lane_solve(const unblending_solver_options& so) { return so.fp64_variant < 0 && so.threads_per_block == 0; }
 
 // Bytes of a global-memory L-BFGS history array for L layers and values of
 // `elem` bytes, sized for kGlobalHistoryBlocksPerSm blocks on every SM.
@@ -686,7 +684,7 @@ PassResult enqueue_pass(Context& c, const Spec& sp, bool refine, const unblendin
     // One history array serves the FP32 solve and the FP64 re-solve (they run
     // one after the other on the stream).
     const int solved = io.pixel_count >= 0 ? io.pixel_count : int(n);
-    const bool lanes = lane_solve(so, L, refine, solved);
+    const bool lanes = lane_solve(so);
     const int v64 = lanes ? kFp64Lanes : fp64_variant(so, refine);
     // (the FP32 solve's global history, where its variant has one, is of the quads' size)
     const size_t quad_history = lanes && so.precision == UNBLENDING_PRECISION_FP64 ? 0 : history_bytes(L, sizeof(double), c.sms);
@@ -1195,7 +1193,7 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
                 if (so.precision == UNBLENDING_PRECISION_FP64 && G.infer.empty()) a.miss_count = G.counts + 1;
                 plan->counts.push_back(G.counts);
                 plan->pixels += total;
-                const bool lanes = lane_solve(so, L, false, total);
+                const bool lanes = lane_solve(so);
                 G.v64 = lanes ? kFp64Lanes : fp64_variant(so, false);
                 const size_t quad_history =
                     lanes && so.precision == UNBLENDING_PRECISION_FP64 ? 0 : history_bytes(L, sizeof(double), c.sms);
