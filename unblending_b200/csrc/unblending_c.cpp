@@ -234,7 +234,7 @@ struct Context {
     Buffer image, first, out, targets, fstatus, scratch, list_a, list_b, small, status, counters, history;
     Buffer order, order_cells;               // work-queue order of a pass (order.cu) and its counting-sort cells
     Buffer defer_list, defer_state;          // pixels deferred by an FP64 solve launch and their state
-    Buffer warm, mlp_w, mlp_b;               // warm-start network on the device
+    Buffer warm, mlp_w, mlp_b, mlp_grad;     // warm-start network on the device, its gradient
     Staging staging;                         // page-locked chunks for pageable caller buffers
     std::vector<float> mlp_uploaded;         // parameters currently in mlp_w / mlp_b
     // Concurrent branches of a batched pass (one per layer-count group) and
@@ -1381,8 +1381,7 @@ int32_t unblending_mlp_loss_grad_device(const unblending_mlp* model, int32_t cou
         cudaStream_t s = c.stream;
         const MlpDevice dev = upload_model(c, *model, s);
         const size_t nw = mlp_weight_count(), nb = mlp_bias_count(), np = nw + nb;
-        Buffer grad_b;
-        float* grad = grad_b.get<float>(np + 1);
+        float* grad = c.mlp_grad.get<float>(np + 1);
         ck(cudaMemsetAsync(grad, 0, (np + 1) * sizeof(float), s));
         MlpGrad g;
         size_t o = 0, ob = nw;
