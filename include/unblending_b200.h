@@ -213,10 +213,10 @@ UNBLENDING_API int32_t unblending_refine_device_rows(
  * loading the library holds until the process exits; images larger than
  * 2048 * 2048 = 4,194,304 pixels return UNBLENDING_INVALID_ARGUMENT, and so
  * does a solver->warm_start (the learned start needs buffers of its own).
- * Kernel variants that keep their L-BFGS history in global memory are
- * replaced by their shared-memory counterparts: the same results, but the
- * FP64 solves run slower than unblending_unmix_device's (about 1.7x on the
- * FP64 re-solve of a 1024x1024 five-layer image). The call
+ * The FP64 solve runs on as many blocks as the array has room for; kernel
+ * variants that would need more are replaced by their shared-memory
+ * counterparts. The results are the same, but the FP64 solves run slower than
+ * unblending_unmix_device's (about 4x on a 1024x1024 five-layer image). The call
  * uses no cudaMalloc, cudaFree, library stream or event; work is enqueued on
  * `stream` (NULL: the legacy default stream) and the call returns without
  * synchronizing. The first call on a device resolves the array's device

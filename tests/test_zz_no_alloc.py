@@ -70,3 +70,17 @@ def test_noalloc_second_image_after_first(cuda):
             np.testing.assert_allclose(out, ref, atol=1e-12, rtol=0)
             assert np.array_equal(status, ref_status)
 
+
+
+@pytest.mark.parametrize("precision,size", [(1, (700, 500)), (0, (1700, 1300)), (0, (2048, 2048))])
+def test_noalloc_sizes_of_the_records(cuda, precision, size):
+    """The array's room for the lanes' records: the FP64 precision at a size
+    that refills its lanes many times, the FP32 precision's re-solve with the
+    lists taking half of it (lanes) and all of it (quads)."""
+    import torch
+    from unblending_b200 import synthetic as syn
+    wl = syn.generate(*size, [0, 1], (20.0, 60.0), seed=61)
+    ref, ref_status, outs = _run(cuda, torch, wl, cuda.solver_options(precision=precision))
+    for out, status in outs:
+        np.testing.assert_array_equal(out, ref)
+        assert np.array_equal(status, ref_status)

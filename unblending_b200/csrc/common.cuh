@@ -89,9 +89,8 @@ __host__ __device__ constexpr int lane_smem_bytes(int L) {
 // registers instead of 168, spilled 600 bytes and was slower).
 __host__ __device__ constexpr int lane_blocks_per_sm(int L) { return L <= 4 ? 4 : L <= 6 ? 3 : 2; }
 __host__ __device__ constexpr int lane_blocks(int L, int sms) { return lane_blocks_per_sm(L) * sms; }
-__host__ __device__ constexpr size_t lane_history_bytes(int L, int sms) {
-    return size_t(lane_blocks(L, sms)) * kLaneBlock * 32 * size_t(lane_records(L));
-}
+__host__ __device__ constexpr size_t lane_block_bytes(int L) { return size_t(kLaneBlock) * 32 * size_t(lane_records(L)); }
+__host__ __device__ constexpr size_t lane_history_bytes(int L, int sms) { return size_t(lane_blocks(L, sms)) * lane_block_bytes(L); }
 
 // Words a lane of a deferred pixel keeps (SolveArgs::defer_state): x, the
 // best point and the start seed (L each), up to L multipliers, and seven

@@ -1595,11 +1595,26 @@ int32_t unblending_unmix_device_noalloc(int32_t width, int32_t height, const dou
         a.miss_list = list_a;
         a.miss_count = counts + 0;
         const int threads = so.threads_per_block ? so.threads_per_block : 128;
-        // Kernel variants that keep their history in global memory would need
-        // an array: this entry point runs their shared-memory counterparts
-        // (same results).
-        const int v64 = variant_global_history(true, fp64_variant(so, false)) ? 0 : fp64_variant(so, false);
-        if (so.precision == UNBLENDING_PRECISION_FP64) {
+        // The FP64 solve runs one pixel per lane on as many blocks as the rest of
+        // the array has records for (at five layers 99 of the 444 that fill the
+        // GPU; the FP64 precision needs no lists): 400x300 pixels, three / five /
+        // eight layers, 9.7 / 49 / 116 -> 7.1 / 29 / 48 ms against the quad kernel
+        // with its history in shared memory. That kernel (same results) serves
+        // quad variants, which would need an array of their own, and re-solves
+        // whose lists leave too little room.
+        const bool fp64 = so.precision == UNBLENDING_PRECISION_FP64;
+        const size_t lists = fp64 ? 0 : (2 * n * sizeof(int32_t) + 255) / 256 * 256;
+        const int lane_block_count = int(std::min<size_t>(size_t(lane_blocks(L, sms)),
+                                                          (bytes - 256 - lists) / lane_block_bytes(L)));
+        const bool lanes = lane_solve(so) && lane_block_count >= sms / 4;
+        const int v64 = lanes ? kFp64Lanes : variant_global_history(true, fp64_variant(so, false)) ? 0 : fp64_variant(so, false);
+        auto attach_fp64 = [&](SolveArgs& x) {
+            if (!lanes) return;
+            x.history = static_cast<unsigned char*>(base) + 256 + lists;
+            x.history_lanes = lane_block_count * kLaneBlock;
+        };
+        if (fp64) {
+            if (lanes) { a.miss_list = nullptr; attach_fp64(a); }
             ck(launch_solve_fp64(L, false, v64, make_models<double>(layers, L), ctl, a, threads, sms, s));
             ++t_launches;
         } else {
@@ -1612,6 +1627,7 @@ int32_t unblending_unmix_device_noalloc(int32_t width, int32_t height, const dou
                 b.list = list_a; b.list_count = counts + 0;
                 b.miss_list = list_b; b.miss_count = counts + 1;
                 b.queue = queues + 1;
+                attach_fp64(b);
                 ck(launch_solve_fp64(L, false, v64, make_models<double>(layers, L), ctl_re, b, threads, sms, s));
                 ++t_launches;
             }
