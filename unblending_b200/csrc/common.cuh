@@ -79,15 +79,16 @@ __host__ __device__ constexpr int lane_records(int L) { return (2 * kLaneRing + 
 // Shared memory of a lane in 16-byte units: x, g, d (4 L values each; d's area
 // also takes the two-loop recursion's coefficients, six pairs).
 __host__ __device__ constexpr int lane_smem_units(int L) { return 4 * L + (2 * L > kHistory ? 2 * L : kHistory); }
-__host__ __device__ constexpr bool lane_shared_targets(int L) { return L != 6; }
+constexpr int kLaneExtra = 14;   // doubles a lane of the solver's scalars
 __host__ __device__ constexpr int lane_smem_bytes(int L) {
-    return lane_smem_units(L) * kLaneBlock * 16 + (lane_shared_targets(L) ? 7 * kLaneBlock * 8 : 0);
+    return lane_smem_units(L) * kLaneBlock * 16 + kLaneExtra * kLaneBlock * 8;
 }
-// Resident blocks per SM: what shared memory holds for many layers (61 KB a
-// block at five layers, 98 KB at eight), and enough registers for the
-// direction's unrolled loops for few (a third block more at five layers, 128
-// registers instead of 168, spilled 600 bytes and was slower).
-__host__ __device__ constexpr int lane_blocks_per_sm(int L) { return L <= 4 ? 4 : L <= 6 ? 3 : 2; }
+// Resident blocks per SM: what the registers (168 a thread for three blocks,
+// 255 for two) and shared memory (76 KB a block at five layers, 113 KB at
+// eight) hold. Six layers spill at three blocks and run in 24.3 ms where two
+// take 18.7 (640x480, first pass); four layers and fewer spill at four blocks
+// (38 against 24 ms on 680x834).
+__host__ __device__ constexpr int lane_blocks_per_sm(int L) { return L <= 5 ? 3 : 2; }
 __host__ __device__ constexpr int lane_blocks(int L, int sms) { return lane_blocks_per_sm(L) * sms; }
 __host__ __device__ constexpr size_t lane_block_bytes(int L) { return size_t(kLaneBlock) * 32 * size_t(lane_records(L)); }
 __host__ __device__ constexpr size_t lane_history_bytes(int L, int sms) { return size_t(lane_blocks(L, sms)) * lane_block_bytes(L); }

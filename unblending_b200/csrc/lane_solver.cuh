@@ -23,9 +23,9 @@
 // for them (or none has a trial). With each warp on its own schedule, the
 // instruction cache thrashed between the phases' code (85-100 KB; 4 to 7 cycles
 // of fetch stall per issue, 75 + 45 ms for the two passes of the 1024x1024
-// five-layer image); with the block in phase the stall is 0.3 cycles (42 + 23
+// five-layer image); with the block in phase the stall is 0.3 cycles (34 + 22
 // ms, against 134 + 99 on quads). Even a block whose warps meet once a trip
-// only is slower (46 + 28 ms).
+// only is slower (measured at 42 + 26 ms: 47 + 28).
 //
 // What bounds it (1024x1024, five layers, first pass): latency at three warps
 // per scheduler (the shared memory and registers that a pixel's state and the
@@ -233,7 +233,6 @@ enum : int { kLaneIdle = 0, kLaneTrial, kLaneOuter, kLaneGrad, kLaneDir, kLaneSt
 
 template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     static constexpr int NV = REFINE ? 3 : 4;    // components of a layer that the method moves
-    static constexpr bool kSharedTargets = lane_shared_targets(L);
     const Models<double>* models_;
     const SolverControls& ctl;
     const SolveArgs& a;
@@ -244,8 +243,7 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     // The pixel's state that its trials read. The rest, read once an outer
     // step, is in two records: the constraint residual at x, and `Outer`.
     int state = kLaneFetch;
-    double target_[kSharedTargets ? 1 : 3], lam_[kSharedTargets ? 1 : NV];
-    double rho, f, step, best_norm, best_energy;
+    double rho, f, step;
     double best_step;   // kBestAtTrial: its step along d
     int it, bt, valid, next;
     bool second;        // the line search's steepest-descent attempt
@@ -258,9 +256,7 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     // best point was a fifth of a trial's instructions).
     enum : int { kNoBest = 0, kBestStored, kBestAtX, kBestAtTrial };
     int best_at;
-    // Between the trial phase and the gradient phase of one trip.
-    bool pending = false;
-    double res_kept[NV], ss_kept;
+    bool pending = false;   // the gradient phase of this trip is this lane's too
 
     __device__ LaneSolver(const Models<double>* m, const SolverControls& c, const SolveArgs& args)
         : models_(m), ctl(c), a(args) {
@@ -283,17 +279,21 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         p[kLaneBlock] = make_double2(v2, v3);
     }
     enum : int { kX = 0, kG = 1, kD = 2 };
-    // The target colour and the multipliers: in shared memory where it has
-    // room (seven registers pairs more for the loops), else in registers.
-    __device__ __forceinline__ double& extra(int k) const {
+    // What a trial reads or leaves once: in shared memory, for the registers
+    // that the loops need (at 168 a thread every spilled value is read back
+    // through a first-level cache of 28 KB: the four-layer kernels with 128
+    // registers and a fourth block spilled 600 bytes and took 38 ms where
+    // they take 24).
+    __device__ __forceinline__ static double& extra(int k) {
         return reinterpret_cast<double*>(lane_smem + lane_smem_units(L) * kLaneBlock * 16)[k * kLaneBlock + threadIdx.x];
     }
-    __device__ __forceinline__ double& target(int c) {
-        if constexpr (kSharedTargets) return extra(c); else return target_[c];
-    }
-    __device__ __forceinline__ double& lam(int c) {
-        if constexpr (kSharedTargets) return extra(3 + c); else return lam_[c];
-    }
+    __device__ __forceinline__ static double& target(int c) { return extra(c); }
+    __device__ __forceinline__ static double& lam(int c) { return extra(3 + c); }
+    __device__ __forceinline__ static double& best_norm() { return extra(7); }
+    __device__ __forceinline__ static double& best_energy() { return extra(8); }
+    // From the trial phase to the gradient phase of one trip.
+    __device__ __forceinline__ static double& ss_kept() { return extra(9); }
+    __device__ __forceinline__ static double& res_kept(int c) { return extra(10 + c); }
     // Record k of a lane whose records start at `base`.
     __device__ __forceinline__ static double* rec(double* base, int k) { return base + k * (kLaneBlock * 4); }
     __device__ __forceinline__ static double* ring(double* base, int s, int w, int l) { return rec(base, (s * 2 + w) * L + l); }
@@ -453,9 +453,9 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
             small_change = small_change || !moved;
             if (best_here) best_at = kBestAtX;
             if (best_lost) best_at = kBestStored;
-            ss_kept = sum(ss);
+            ss_kept() = sum(ss);
 #pragma unroll
-            for (int c = 0; c < NV; ++c) res_kept[c] = res[c];
+            for (int c = 0; c < NV; ++c) res_kept(c) = res[c];
             store_rec(residual_rec(), res[0], res[1], res[2], res[NV - 1]);
             return;
         }
@@ -474,9 +474,9 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         const double tol2 = ctl.outer_tolerance * ctl.outer_tolerance;
         const bool feasible = norm < tol2;
         if (isfinite(energy) && isfinite(norm) &&
-            (best_at == kNoBest || (feasible && (best_norm >= tol2 || energy < best_energy)) ||
-             (!feasible && best_norm >= tol2 && norm < best_norm))) {
-            best_norm = norm; best_energy = energy; best_moved = true;
+            (best_at == kNoBest || (feasible && (best_norm() >= tol2 || energy < best_energy())) ||
+             (!feasible && best_norm() >= tol2 && norm < best_norm()))) {
+            best_norm() = norm; best_energy() = energy; best_moved = true;
             best_at = at_x ? kBestAtX : kBestAtTrial;
             best_step = step;
         }
@@ -524,9 +524,9 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         const Models<double>& m = *models_;
         const bool at_x = !from_trial;
         // Reverse sweep; layer l's slot of d turns from its composite into its gradient.
-        double adj[3], adj3 = REFINE ? 0.0 : rho * res_kept[NV - 1] - lam(NV - 1);
+        double adj[3], adj3 = REFINE ? 0.0 : rho * res_kept(NV - 1) - lam(NV - 1);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) adj[c] = rho * res_kept[c] - lam(c);
+        for (int c = 0; c < 3; ++c) adj[c] = rho * res_kept(c) - lam(c);
 #pragma unroll 1
         for (int l = L - 1; l >= 0; --l) {
             double t[4], ng[4];
@@ -623,7 +623,7 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         }
         double yyt = sum(yy);
         if (REFINE) yyt += ya;
-        if (curvature(sum(sy), ss_kept, yyt)) {
+        if (curvature(sum(sy), ss_kept(), yyt)) {
             next = next + 1 == kLaneRing ? 0 : next + 1;
             valid = valid + 1 < kHistory ? valid + 1 : kHistory;
         }
@@ -660,11 +660,10 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         state = kLaneTrial;
     }
 
-    // Forms d from x, g and the ring. Out of line, so that the unrolled loops
-    // have the registers to themselves (the caller's state goes to the stack
-    // once per call).
+    // Forms d from x, g and the ring (static: it touches none of the pixel's
+    // other state).
     enum : int { kStationary = 0, kFormed = 1, kReset = 2 };
-    __device__ __noinline__ static int form_direction(double* base, int valid, int next, bool steep, bool opaque,
+    __device__ __forceinline__ static int form_direction(double* base, int valid, int next, bool steep, bool opaque,
                                                       bool smooth, bool finite_f) {
         uint32_t freem = 0;
         {
@@ -991,8 +990,8 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
             if (a.input_failed) atomicAdd(a.input_failed, 1);
             return;
         }
-        if (best_at == kNoBest) best_norm = written_norm(*models_, outp, image(o) + 3 * i, n, i);
-        const bool miss = !(best_norm < ctl.outer_tolerance * ctl.outer_tolerance);
+        if (best_at == kNoBest) best_norm() = written_norm(*models_, outp, image(o) + 3 * i, n, i);
+        const bool miss = !(best_norm() < ctl.outer_tolerance * ctl.outer_tolerance);
         if (stp) stp[i] = miss ? 3 : 0;
         if (miss && a.miss_list) a.miss_list[atomicAdd(a.miss_count, 1)] = int32_t(o.gidx);
     }
@@ -1046,7 +1045,7 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
 #pragma unroll
         for (int c = 0; c < 3; ++c) target(c) = p[c];
         best_at = kNoBest;
-        best_norm = INFINITY; best_energy = INFINITY;
+        best_norm() = INFINITY; best_energy() = INFINITY;
         if (a.counters)
 #pragma unroll
             for (int k = 0; k < 5; ++k) a.counters[5 * size_t(o.gidx) + k] = 0;

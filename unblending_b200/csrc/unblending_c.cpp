@@ -458,9 +458,9 @@ int fp64_variant(const unblending_solver_options& so, bool refine) {
 // the smallest launches (a launch spreads its pixels over all warps) and by
 // throughput in the large ones. Lanes / quads, ms, first pass and refinement:
 // three layers, 64 pixels 0.6 / 0.8 and 0.3 / 0.7, 5,184 1.7 / 2.1 and 1.5 / 3.0,
-// 65,536 2.3 / 4.1 and 2.0 / 4.6; five layers, 576 2.7 / 4.6 and 2.0 / 6.5, 65,536
-// 6.2 / 12.8 and 4.6 / 12.5; eight layers, 576 3.6 / 9.2 and 3.0 / 9.2, 65,536 11 / 57
-// and 8.7 / 28.
+// 65,536 2.0 / 4.1 and 2.0 / 4.6; five layers, 576 2.7 / 4.6 and 2.0 / 6.5,
+// 1,048,576 34 / 134 and 22 / 99; eight layers, 576 3.6 / 9.2 and 3.0 / 9.2, 65,536
+// 11 / 57 and 8.7 / 28.
 bool lane_solve(const unblending_solver_options& so) { return so.fp64_variant < 0 && so.threads_per_block == 0; }
 
 // Bytes of a global-memory L-BFGS history array for L layers and values of
