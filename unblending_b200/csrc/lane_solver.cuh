@@ -233,6 +233,9 @@ enum : int { kLaneIdle = 0, kLaneTrial, kLaneOuter, kLaneGrad, kLaneDir, kLaneSt
 
 template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     static constexpr int NV = REFINE ? 3 : 4;    // components of a layer that the method moves
+    // The evaluation's layers are unrolled for up to three; at five the code
+    // outgrows the instruction cache (42 -> 48 ms).
+    static constexpr int kUnroll = L <= 3 ? L : 1;
     const Models<double>* models_;
     const SolverControls& ctl;
     const SolveArgs& a;
@@ -406,7 +409,7 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         uint32_t largest = 0;   // high word of the largest motion of a component
 #pragma unroll
         for (int c = 0; c < NV; ++c) { sl[c] = 0.0; ss[c] = 0.0; }
-#pragma unroll 1
+#pragma unroll kUnroll
         for (int l = 0; l < L; ++l) {
             double x[4], d[4], g[4], t[4], s[4] = {0.0, 0.0, 0.0, 0.0};
             get(kX, l, x); get(kD, l, d); get(kG, l, g);
@@ -1061,11 +1064,28 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         // A small launch spreads its pixels over all warps.
         const int warps = int(gridDim.x) * (kLaneBlock / 32);
         if (total <= 0 || lane > (total - 1) / warps) state = kLaneIdle;
+        // Lanes waiting for each phase, one byte a phase (trial, direction,
+        // gradient, outer step), counted over the block with one barrier, in
+        // two buffers in turn.
+        __shared__ uint32_t counts[2][kLaneBlock / 32];
+        int turn = 0, nf = 0, nd = 0, nb = 0, ne = 0, live = 0;
+        auto recount = [&]() {
+            const uint32_t mine = uint32_t(__popc(__ballot_sync(full, state == kLaneTrial || state == kLaneOuter))) |
+                                  uint32_t(__popc(__ballot_sync(full, state == kLaneDir || state == kLaneSteep))) << 8 |
+                                  uint32_t(__popc(__ballot_sync(full, state == kLaneGrad))) << 16 |
+                                  uint32_t(__popc(__ballot_sync(full, state == kLaneEnd || state == kLaneFetch))) << 24;
+            if (lane == 0) counts[turn][threadIdx.x >> 5] = mine;
+            __syncthreads();
+            uint32_t all = 0;
+#pragma unroll
+            for (int w = 0; w < kLaneBlock / 32; ++w) all += counts[turn][w];
+            nf = all & 255; nd = all >> 8 & 255; nb = all >> 16 & 255; ne = all >> 24;
+            live = nf + nd + nb + ne;
+            turn ^= 1;
+        };
         for (;;) {
-            const int live = __syncthreads_count(state != kLaneIdle);
+            recount();
             if (live == 0) break;
-            const int ne = __syncthreads_count(state == kLaneEnd || state == kLaneFetch);
-            int nf = __syncthreads_count(state == kLaneTrial || state == kLaneOuter);
             if (ne > 0 && (8 * ne >= kOuterQuorum * live || nf == 0)) {
                 int what = kFinished;
                 bool write = false, skipped = false;
@@ -1098,16 +1118,13 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
                     if (what == kNextStart) begin_start(o);
                     begin_outer(o);
                 }
+                __syncwarp();
+                recount();
             }
-            __syncwarp();
-            nf = __syncthreads_count(state == kLaneTrial || state == kLaneOuter);
-            const int nd = __syncthreads_count(state == kLaneDir || state == kLaneSteep);
             if (nd > 0 && (8 * nd >= kDirectionQuorum * live || nf == 0)) {
                 if (state == kLaneDir || state == kLaneSteep) direction();
-                __syncwarp();
+                recount();
             }
-            nf = __syncthreads_count(state == kLaneTrial || state == kLaneOuter);
-            const int nb = __syncthreads_count(state == kLaneGrad);
             const bool gradients = nb > 0 && (8 * nb >= kGradientQuorum * live || nf == 0);
             if (state == kLaneTrial || state == kLaneOuter || (gradients && state == kLaneGrad)) {
                 const bool mine = state == kLaneGrad;
