@@ -42,7 +42,8 @@ typedef struct unblending_solver_options {
     double inner_tolerance;     /* default 5e-3 */
     double outer_tolerance;     /* feasibility tolerance on |C|, default 5e-3 */
     int32_t threads_per_block;  /* 0 selects the tuned default */
-    int32_t kernel_variant;     /* FP32 solve: -1 tuned default; 0 history in registers; 1/2 history in shared
+    int32_t kernel_variant;     /* FP32 solve: -1 default, one pixel per lane (batches: a tuned quad variant);
+                                   quad variants: 0 history in registers; 1/2 history in shared
                                    memory with registers capped for 4/5 blocks per SM; 3 as 1 with the evaluation
                                    rolled over the layers; 4 history in global memory, rolled, 5 blocks per SM;
                                    5 as 3, with three lanes per pixel where the alphas are pinned (refinement) */

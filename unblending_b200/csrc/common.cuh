@@ -69,29 +69,37 @@ struct SolverControls {
 };
 
 // Lane kernels (lane_solver.cuh), one pixel per lane: blocks of four warps.
-// A lane's global-memory records (32 bytes: one layer's three colours and
-// alpha) are the steps and gradient changes of the L-BFGS ring, which has a
+// A lane's global-memory records (32 bytes, in FP32 16: one layer's three
+// colours and alpha) are the steps and gradient changes of the L-BFGS ring, which has a
 // spare slot that an accepted step fills before its curvature test, the best
 // point, the outer step's start, and two of what an outer step keeps.
 constexpr int kLaneBlock = 128;
 constexpr int kLaneRing = kHistory + 1;
-__host__ __device__ constexpr int lane_records(int L) { return (2 * kLaneRing + 2) * L + 2; }
+__host__ __device__ constexpr int lane_records(int L, bool fp32) { return (2 * kLaneRing + 2) * L + (fp32 ? 3 : 2); }
 // Shared memory of a lane in 16-byte units: x, g, d (4 L values each; d's area
 // also takes the two-loop recursion's coefficients, six pairs).
-__host__ __device__ constexpr int lane_smem_units(int L) { return 4 * L + (2 * L > kHistory ? 2 * L : kHistory); }
-constexpr int kLaneExtra = 14;   // doubles a lane of the solver's scalars
-__host__ __device__ constexpr int lane_smem_bytes(int L) {
-    return lane_smem_units(L) * kLaneBlock * 16 + kLaneExtra * kLaneBlock * 8;
+__host__ __device__ constexpr int lane_smem_units(int L, bool fp32) {
+    return fp32 ? 2 * L + (L > kHistory ? L : kHistory) : 4 * L + (2 * L > kHistory ? 2 * L : kHistory);
 }
-// Resident blocks per SM: what the registers (168 a thread for three blocks,
+constexpr int kLaneExtra = 14;   // doubles a lane of the solver's scalars
+__host__ __device__ constexpr int lane_smem_bytes(int L, bool fp32) {
+    return lane_smem_units(L, fp32) * kLaneBlock * 16 + kLaneExtra * kLaneBlock * (fp32 ? 4 : 8);
+}
+// Resident blocks per SM. FP64: what the registers (168 a thread for three blocks,
 // 255 for two) and shared memory (76 KB a block at five layers, 113 KB at
 // eight) hold. Six layers spill at three blocks and run in 24.3 ms where two
 // take 18.7 (640x480, first pass); four layers and fewer spill at four blocks
-// (38 against 24 ms on 680x834).
-__host__ __device__ constexpr int lane_blocks_per_sm(int L) { return L <= 5 ? 3 : 2; }
-__host__ __device__ constexpr int lane_blocks(int L, int sms) { return lane_blocks_per_sm(L) * sms; }
-__host__ __device__ constexpr size_t lane_block_bytes(int L) { return size_t(kLaneBlock) * 32 * size_t(lane_records(L)); }
-__host__ __device__ constexpr size_t lane_history_bytes(int L, int sms) { return size_t(lane_blocks(L, sms)) * lane_block_bytes(L); }
+// (38 against 24 ms on 680x834). FP32, 1024x1024 five layers, first pass +
+// refinement in ms by blocks per SM: three 23.1 + 16.4, four 20.0 + 13.9, five
+// 21.3 + 15.5, six 26.4 + 16.6 (spills).
+__host__ __device__ constexpr int lane_blocks_per_sm(int L, bool fp32) { return fp32 ? (L <= 6 ? 4 : 3) : L <= 5 ? 3 : 2; }
+__host__ __device__ constexpr int lane_blocks(int L, int sms, bool fp32) { return lane_blocks_per_sm(L, fp32) * sms; }
+__host__ __device__ constexpr size_t lane_block_bytes(int L, bool fp32) {
+    return size_t(kLaneBlock) * (fp32 ? 16 : 32) * size_t(lane_records(L, fp32));
+}
+__host__ __device__ constexpr size_t lane_history_bytes(int L, int sms, bool fp32) {
+    return size_t(lane_blocks(L, sms, fp32)) * lane_block_bytes(L, fp32);
+}
 
 // Words a lane of a deferred pixel keeps (SolveArgs::defer_state): x, the
 // best point and the start seed (L each), up to L multipliers, and seven

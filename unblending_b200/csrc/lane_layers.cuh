@@ -1,5 +1,5 @@
-// Lane kernels (one pixel per lane, FP64) of one layer count, UNB_SOLVER_LAYERS:
-// first pass, batched first pass and refinement. Included by lane_l<L>.cu,
+// Lane kernels (one pixel per lane) of one layer count, UNB_SOLVER_LAYERS: first
+// pass and refinement in FP64 and FP32, batched first pass in FP64. Included by lane_l<L>.cu,
 // which are compiled with --fmad=false as the other solve kernels are.
 #include <algorithm>
 
@@ -15,11 +15,11 @@ namespace unb {
 namespace {
 constexpr int kL = UNB_SOLVER_LAYERS;
 
-template <bool R, bool BATCH>
-cudaError_t lanes(const Models<double>& m, const SolverControls& c, const SolveArgs& a, int sms, cudaStream_t s) {
-    auto k = solve_lanes<kL, R, BATCH>;
+template <class T, bool R, bool BATCH>
+cudaError_t lanes(const Models<T>& m, const SolverControls& c, const SolveArgs& a, int sms, cudaStream_t s) {
+    auto k = solve_lanes<T, kL, R, BATCH>;
     if (!a.history) return cudaErrorInvalidValue;
-    constexpr int smem = lane_smem_bytes(kL);
+    constexpr int smem = lane_smem_bytes(kL, sizeof(T) == 4);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
@@ -35,8 +35,13 @@ cudaError_t lanes(const Models<double>& m, const SolverControls& c, const SolveA
 
 template <> cudaError_t solve_lanes_layers<kL>(bool refine, bool batch, const Models<double>& m, const SolverControls& c,
                                                const SolveArgs& a, int sms, cudaStream_t s) {
-    if (batch) return lanes<false, true>(m, c, a, sms, s);
-    return refine ? lanes<true, false>(m, c, a, sms, s) : lanes<false, false>(m, c, a, sms, s);
+    if (batch) return lanes<double, false, true>(m, c, a, sms, s);
+    return refine ? lanes<double, true, false>(m, c, a, sms, s) : lanes<double, false, false>(m, c, a, sms, s);
+}
+
+template <> cudaError_t solve_lanes_fp32_layers<kL>(bool refine, const Models<float>& m, const SolverControls& c,
+                                                    const SolveArgs& a, int sms, cudaStream_t s) {
+    return refine ? lanes<float, true, false>(m, c, a, sms, s) : lanes<float, false, false>(m, c, a, sms, s);
 }
 
 }  // namespace unb

@@ -1,10 +1,10 @@
-// Per-pixel augmented-Lagrangian / projected L-BFGS solve, one pixel per lane
-// (FP64).
+// Per-pixel augmented-Lagrangian / projected L-BFGS solve, one pixel per lane.
 //
-// The method, its FP64 arithmetic and its operation order are those of
-// solver.cuh (rounded multiplies and adds; a pixel's sums over the three
-// channels and the alphas are added in the tree in which a quad's lanes add
-// theirs), so outputs, statuses and counters equal its kernels' bit for bit.
+// The method, its arithmetic and its operation order are those of solver.cuh
+// (FP64: rounded multiplies and adds; FP32: its fused and approximate forms; a
+// pixel's sums over the three channels and the alphas are added in the tree in
+// which a quad's lanes add theirs), so outputs, statuses and counters equal
+// its kernels' bit for bit in both precisions. Figures below are FP64's.
 //
 // Why one pixel per lane: on a quad, all four lanes repeat the composite alpha
 // chain and the 3x3 colour prior, lane 3 idles through the colour arithmetic,
@@ -55,8 +55,6 @@ __device__ __forceinline__ double reciprocal(double b) {
     const bool ones = (uint32_t(__double2hiint(b)) | 0xfff00000u) == 0xffffffffu && __double2loint(b) == -1;
     return __hiloint2double(__double2hiint(y), ones ? 1 : __double2loint(y));
 }
-
-__device__ __forceinline__ double mul_add(double a, double b, double c) { return __dadd_rn(__dmul_rn(a, b), c); }
 
 // Blend values of three channels of one layer (blend_value of each).
 __device__ __forceinline__ void blend_value3(int mode, const double* s, const double* d, double* f) {
@@ -211,6 +209,25 @@ __device__ __forceinline__ void blend_all3(int mode, const double* s, const doub
     }
 }
 
+// FP32: the solver's table-driven blends, channel by channel.
+__device__ __forceinline__ void blend_values(const Models<float>& m, int l, const float* s, const float* d, float* f) {
+    float fs, fd;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) blend_table<float>(m, l, s[c], d[c], f[c], fs, fd, false);
+}
+__device__ __forceinline__ void blend_all(const Models<float>& m, int l, const float* s, const float* d, float* f,
+                                          float* fs, float* fd) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) blend_table<float>(m, l, s[c], d[c], f[c], fs[c], fd[c], true);
+}
+__device__ __forceinline__ void blend_values(const Models<double>& m, int l, const double* s, const double* d, double* f) {
+    blend_value3(m.mode[l], s, d, f);
+}
+__device__ __forceinline__ void blend_all(const Models<double>& m, int l, const double* s, const double* d, double* f,
+                                          double* fs, double* fd) {
+    blend_all3(m.mode[l], s, d, f, fs, fd);
+}
+
 // ----------------------------------------------------------------- storage --
 // A lane's four values of one layer (three colours, alpha) as one 32-byte
 // sector of global memory.
@@ -222,6 +239,17 @@ __device__ __forceinline__ void store_rec(double* p, double a, double b, double 
     asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
 }
 
+__device__ __forceinline__ void load_rec(const float* p, float* v) {
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void store_rec(float* p, float a, float b, float c, float d) {
+    asm volatile("st.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+// Bits of the magnitude (double: of its high word), ordered as magnitudes are.
+__device__ __forceinline__ uint32_t magnitude_bits(double v) { return uint32_t(__double2hiint(v)) & 0x7fffffffu; }
+__device__ __forceinline__ uint32_t magnitude_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+
 extern __shared__ __align__(16) unsigned char lane_smem[];
 
 // Eighths of a block's live lanes that start a phase: the end of an outer
@@ -231,23 +259,24 @@ extern __shared__ __align__(16) unsigned char lane_smem[];
 constexpr int kOuterQuorum = 2, kDirectionQuorum = 2, kGradientQuorum = 2;
 enum : int { kLaneIdle = 0, kLaneTrial, kLaneOuter, kLaneGrad, kLaneDir, kLaneSteep, kLaneEnd, kLaneFetch };
 
-template <int L, bool REFINE, bool BATCH> struct LaneSolver {
+template <class T, int L, bool REFINE, bool BATCH> struct LaneSolver {
+    static constexpr bool kFast = sizeof(T) == 4;   // the FP32 solver's arithmetic: fused, approximate division
     static constexpr int NV = REFINE ? 3 : 4;    // components of a layer that the method moves
     // The evaluation's layers are unrolled for up to three; at five the code
     // outgrows the instruction cache (42 -> 48 ms).
     static constexpr int kUnroll = L <= 3 ? L : 1;
-    const Models<double>* models_;
+    const Models<T>* models_;
     const SolverControls& ctl;
     const SolveArgs& a;
     const int lane = threadIdx.x & 31;
-    double* rec_base;       // this lane's records, kLaneBlock apart: a block's are contiguous
+    T* rec_base;       // this lane's records, kLaneBlock apart: a block's are contiguous
     uint32_t n_value = 0, n_grad = 0;
 
     // The pixel's state that its trials read. The rest, read once an outer
     // step, is in two records: the constraint residual at x, and `Outer`.
     int state = kLaneFetch;
-    double rho, f, step;
-    double best_step;   // kBestAtTrial: its step along d
+    T rho, f, step;
+    T best_step;   // kBestAtTrial: its step along d
     int it, bt, valid, next;
     bool second;        // the line search's steepest-descent attempt
     bool from_trial;    // kLaneGrad: the point is an accepted trial (else the outer step's start)
@@ -261,25 +290,36 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     int best_at;
     bool pending = false;   // the gradient phase of this trip is this lane's too
 
-    __device__ LaneSolver(const Models<double>* m, const SolverControls& c, const SolveArgs& args)
+    __device__ LaneSolver(const Models<T>* m, const SolverControls& c, const SolveArgs& args)
         : models_(m), ctl(c), a(args) {
-        rec_base = static_cast<double*>(a.history) + (size_t(blockIdx.x) * lane_records(L) * kLaneBlock + threadIdx.x) * 4;
-        if constexpr (BATCH) models_ = static_cast<const Models<double>*>(a.models);
+        rec_base = static_cast<T*>(a.history) + (size_t(blockIdx.x) * lane_records(L, kFast) * kLaneBlock + threadIdx.x) * 4;
+        if constexpr (BATCH) models_ = static_cast<const Models<T>*>(a.models);
     }
 
     // ------------------------------------------------------------ storage --
+    // A layer's four values of a lane: two 16-byte units (FP64) or one (FP32).
+    static constexpr int kUnits = kFast ? 1 : 2;
     __device__ __forceinline__ static double2* slot(int unit) {
         return reinterpret_cast<double2*>(lane_smem) + unit * kLaneBlock + threadIdx.x;
     }
-    __device__ __forceinline__ static void get(int vec, int l, double* v) {
-        const double2* p = slot(vec * 2 * L + 2 * l);
-        const double2 u = p[0], w = p[kLaneBlock];
-        v[0] = u.x; v[1] = u.y; v[2] = w.x; v[3] = w.y;
+    __device__ __forceinline__ static void get(int vec, int l, T* v) {
+        const double2* p = slot((vec * L + l) * kUnits);
+        if constexpr (kFast) {
+            const float4 u = *reinterpret_cast<const float4*>(p);
+            v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+        } else {
+            const double2 u = p[0], w = p[kLaneBlock];
+            v[0] = u.x; v[1] = u.y; v[2] = w.x; v[3] = w.y;
+        }
     }
-    __device__ __forceinline__ static void put(int vec, int l, double v0, double v1, double v2, double v3) {
-        double2* p = slot(vec * 2 * L + 2 * l);
-        p[0] = make_double2(v0, v1);
-        p[kLaneBlock] = make_double2(v2, v3);
+    __device__ __forceinline__ static void put(int vec, int l, T v0, T v1, T v2, T v3) {
+        double2* p = slot((vec * L + l) * kUnits);
+        if constexpr (kFast) {
+            *reinterpret_cast<float4*>(p) = make_float4(v0, v1, v2, v3);
+        } else {
+            p[0] = make_double2(v0, v1);
+            p[kLaneBlock] = make_double2(v2, v3);
+        }
     }
     enum : int { kX = 0, kG = 1, kD = 2 };
     // What a trial reads or leaves once: in shared memory, for the registers
@@ -287,48 +327,59 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     // through a first-level cache of 28 KB: the four-layer kernels with 128
     // registers and a fourth block spilled 600 bytes and took 38 ms where
     // they take 24).
-    __device__ __forceinline__ static double& extra(int k) {
-        return reinterpret_cast<double*>(lane_smem + lane_smem_units(L) * kLaneBlock * 16)[k * kLaneBlock + threadIdx.x];
+    __device__ __forceinline__ static T& extra(int k) {
+        return reinterpret_cast<T*>(lane_smem + lane_smem_units(L, kFast) * kLaneBlock * 16)[k * kLaneBlock + threadIdx.x];
     }
-    __device__ __forceinline__ static double& target(int c) { return extra(c); }
-    __device__ __forceinline__ static double& lam(int c) { return extra(3 + c); }
-    __device__ __forceinline__ static double& best_norm() { return extra(7); }
-    __device__ __forceinline__ static double& best_energy() { return extra(8); }
+    __device__ __forceinline__ static T& target(int c) { return extra(c); }
+    __device__ __forceinline__ static T& lam(int c) { return extra(3 + c); }
+    __device__ __forceinline__ static T& best_norm() { return extra(7); }
+    __device__ __forceinline__ static T& best_energy() { return extra(8); }
     // From the trial phase to the gradient phase of one trip.
-    __device__ __forceinline__ static double& ss_kept() { return extra(9); }
-    __device__ __forceinline__ static double& res_kept(int c) { return extra(10 + c); }
+    __device__ __forceinline__ static T& ss_kept() { return extra(9); }
+    __device__ __forceinline__ static T& res_kept(int c) { return extra(10 + c); }
     // Record k of a lane whose records start at `base`.
-    __device__ __forceinline__ static double* rec(double* base, int k) { return base + k * (kLaneBlock * 4); }
-    __device__ __forceinline__ static double* ring(double* base, int s, int w, int l) { return rec(base, (s * 2 + w) * L + l); }
-    __device__ __forceinline__ double* ring(int s, int w, int l) const { return ring(rec_base, s, w, l); }
-    __device__ __forceinline__ double* best_rec(int l) const { return rec(rec_base, 2 * kLaneRing * L + l); }
-    __device__ __forceinline__ double* ox_rec(int l) const { return rec(rec_base, (2 * kLaneRing + 1) * L + l); }
-    __device__ __forceinline__ double* residual_rec() const { return rec(rec_base, (2 * kLaneRing + 2) * L); }
-    __device__ __forceinline__ double* outer_rec() const { return rec(rec_base, (2 * kLaneRing + 2) * L + 1); }
+    __device__ __forceinline__ static T* rec(T* base, int k) { return base + k * (kLaneBlock * 4); }
+    __device__ __forceinline__ static T* ring(T* base, int s, int w, int l) { return rec(base, (s * 2 + w) * L + l); }
+    __device__ __forceinline__ T* ring(int s, int w, int l) const { return ring(rec_base, s, w, l); }
+    __device__ __forceinline__ T* best_rec(int l) const { return rec(rec_base, 2 * kLaneRing * L + l); }
+    __device__ __forceinline__ T* ox_rec(int l) const { return rec(rec_base, (2 * kLaneRing + 1) * L + l); }
+    __device__ __forceinline__ T* residual_rec() const { return rec(rec_base, (2 * kLaneRing + 2) * L); }
+    __device__ __forceinline__ T* outer_rec() const { return rec(rec_base, (2 * kLaneRing + 2) * L + 1); }
 
     // What the method keeps of a pixel between its outer steps.
     struct Outer {
-        double oldnorm;     // squared residual at the outer step's start
+        T oldnorm;     // squared residual at the outer step's start
         int outer, frozen, pixel, gidx, start, job;
     };
     __device__ __forceinline__ Outer load_outer() const {
-        double v[4];
+        T v[4];
         load_rec(outer_rec(), v);
-        return Outer{v[0], __double2hiint(v[1]), __double2loint(v[1]), __double2hiint(v[2]), __double2loint(v[2]),
-                     __double2hiint(v[3]), __double2loint(v[3])};
+        if constexpr (kFast) {
+            T w[4];
+            load_rec(outer_rec() + kLaneBlock * 4, w);
+            return Outer{v[0], __float_as_int(v[1]), __float_as_int(v[2]), __float_as_int(v[3]), __float_as_int(w[0]),
+                         __float_as_int(w[1]), __float_as_int(w[2])};
+        } else {
+            return Outer{v[0], __double2hiint(v[1]), __double2loint(v[1]), __double2hiint(v[2]), __double2loint(v[2]),
+                         __double2hiint(v[3]), __double2loint(v[3])};
+        }
     }
     __device__ __forceinline__ void store_outer(const Outer& o) const {
-        store_rec(outer_rec(), o.oldnorm, __hiloint2double(o.outer, o.frozen), __hiloint2double(o.pixel, o.gidx),
-                  __hiloint2double(o.start, o.job));
+        if constexpr (kFast) {
+            store_rec(outer_rec(), o.oldnorm, __int_as_float(o.outer), __int_as_float(o.frozen), __int_as_float(o.pixel));
+            store_rec(outer_rec() + kLaneBlock * 4, __int_as_float(o.gidx), __int_as_float(o.start), __int_as_float(o.job), 0.0f);
+        } else {
+            store_rec(outer_rec(), o.oldnorm, __hiloint2double(o.outer, o.frozen), __hiloint2double(o.pixel, o.gidx),
+                      __hiloint2double(o.start, o.job));
+        }
     }
-
     // Work counters (only when requested).
     __device__ __forceinline__ void count(int k) const { if (a.counters) ++a.counters[5 * size_t(load_outer().gidx) + k]; }
     __device__ __forceinline__ static bool fixed_bounds(bool opaque, bool smooth, int l, int c) {
         return l == 0 && (c == 3 ? opaque : (REFINE && smooth));
     }
-    __device__ __forceinline__ static bool fixed_at(bool opaque, bool smooth, int l, int c, double x, double g) {
-        return fixed_bounds(opaque, smooth, l, c) || (x <= 0.0 && g > 0.0) || (x >= 1.0 && g < 0.0);
+    __device__ __forceinline__ static bool fixed_at(bool opaque, bool smooth, int l, int c, T x, T g) {
+        return fixed_bounds(opaque, smooth, l, c) || (x <= T(0.0) && g > T(0.0)) || (x >= T(1.0) && g < T(0.0));
     }
     // v in [0, 1] (NaN stays NaN), by its bits: the FP64 pipe has the
     // arithmetic, and its compares are as slow as it is.
@@ -337,35 +388,37 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         const bool keep = uint32_t(hi) < 0x3ff00000u || (uint32_t(hi) & 0x7fffffffu) > 0x7ff00000u;
         return __hiloint2double(keep ? hi : (hi < 0 ? 0 : 0x3ff00000), keep ? __double2loint(v) : 0);
     }
+    __device__ __forceinline__ static float clamp01(float v) { return v < 0.0f ? 0.0f : (v > 1.0f ? 1.0f : v); }
 
     // The per-channel partial sums, added as the lanes of a group add theirs.
-    __device__ __forceinline__ static double sum(const double* v) {
+    __device__ __forceinline__ static T sum(const T* v) {
         if constexpr (REFINE) return (v[0] + v[1]) + v[2];
         else return (v[0] + v[1]) + (v[2] + v[3]);
     }
 
     // ------------------------------------------------------------ forward --
     // One layer of the composite: A, pc in/out.
-    __device__ __forceinline__ void compose(const Models<double>& m, int l, const double* t, double av, double& A,
-                                            double* pc) const {
+    __device__ __forceinline__ void compose(const Models<T>& m, int l, const T* t, T av, T& A,
+                                            T* pc) const {
         if (l == 0) {
             A = av;
 #pragma unroll
             for (int c = 0; c < 3; ++c) pc[c] = t[c];
             return;
         }
-        const double dd = A, X = m.fX[l], Y = m.fY[l], Z = m.fZ[l];
-        const double n_dd = 1.0 - dd, n_av = 1.0 - av;
-        const double ya = __dmul_rn(Y * av, n_dd), zd = __dmul_rn(Z * dd, n_av);
-        const double Al = __dadd_rn(zd, mul_add(X * av, dd, ya));
-        const double y = reciprocal(Al);
-        double fv[3];
-        blend_value3(m.mode[l], t, pc, fv);
-        const bool big = Al > 1e-12;
+        const T dd = A, X = m.fX[l], Y = m.fY[l], Z = m.fZ[l];
+        const T n_dd = T(1.0) - dd, n_av = T(1.0) - av;
+        const T ya = Y * av * n_dd, zd = Z * dd * n_av;
+        const T Al = madd<T>(Z * dd, n_av, madd<T>(X * av, dd, ya));
+        T fv[3], y = T(0);
+        if constexpr (!kFast) y = reciprocal(Al);
+        blend_values(m, l, t, pc, fv);
+        const bool big = Al > T(1e-12);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const double pre = mul_add(zd, pc[c], mul_add(fv[c] * av, dd, ya * t[c]));
-            const double q = quotient(pre, Al, y);
+            const T pre = madd<T>(zd, pc[c], madd<T>(fv[c] * av, dd, ya * t[c]));
+            T q;
+            if constexpr (kFast) q = qdiv(pre, Al); else q = quotient(pre, Al, y);
             pc[c] = big ? q : pre;
         }
         A = Al;
@@ -373,9 +426,9 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
 
     // Point of layer l at step s along d, within bounds (the fixed values have
     // d = 0 and x in [0, 1]; at the start of an outer step d is zero).
-    __device__ __forceinline__ static void point(const double* x, const double* d, double s, double* t) {
+    __device__ __forceinline__ static void point(const T* x, const T* d, T s, T* t) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) t[c] = REFINE && c == 3 ? x[c] : clamp01(mul_add(s, d[c], x[c]));
+        for (int c = 0; c < 4; ++c) t[c] = REFINE && c == 3 ? x[c] : clamp01(madd<T>(s, d[c], x[c]));
     }
 
     // Writes the best point to its records before x or d changes.
@@ -383,7 +436,7 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         const bool at_x = best_at == kBestAtX;
 #pragma unroll 1
         for (int l = 0; l < L; ++l) {
-            double x[4], d[4], t[4];
+            T x[4], d[4], t[4];
             get(kX, l, x); get(kD, l, d);
             point(x, d, best_step, t);
             store_rec(best_rec(l), at_x ? x[0] : t[0], at_x ? x[1] : t[1], at_x ? x[2] : t[2], at_x ? x[3] : t[3]);
@@ -398,50 +451,51 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     // x becomes the accepted point, its step goes to the ring's free slot, and
     // d's slots take the composite's colours and alpha.
     __device__ __forceinline__ void forward() {
-        const Models<double>& m = *models_;
+        const Models<T>& m = *models_;
         const bool keep = state == kLaneGrad, at_x = state == kLaneOuter || (keep && !from_trial);
         // (keep) the accepted point is the best point; the best point is lost with x and d.
         const bool best_here = best_at == kBestAtTrial && best_step == step;
         const bool best_lost = !at_x && (best_at == kBestAtX || (best_at == kBestAtTrial && !best_here));
         bool moved = false;     // (keep) some component moved by at least the inner tolerance
-        const double tol_lo = ctl.inner_tolerance * (1.0 - 0x1p-48), tol_hi = ctl.inner_tolerance * (1.0 + 0x1p-48);
-        double sl[NV], ss[NV], A = 0.0, pc[3], energy = 0.0, asum = 0.0;
+        [[maybe_unused]] const T tol_lo = ctl.inner_tolerance * (1.0 - 0x1p-48), tol_hi = ctl.inner_tolerance * (1.0 + 0x1p-48);
+        T sl[NV], ss[NV], A = T(0.0), pc[3], energy = T(0.0), asum = T(0.0);
         uint32_t largest = 0;   // high word of the largest motion of a component
 #pragma unroll
-        for (int c = 0; c < NV; ++c) { sl[c] = 0.0; ss[c] = 0.0; }
+        for (int c = 0; c < NV; ++c) { sl[c] = T(0.0); ss[c] = T(0.0); }
 #pragma unroll kUnroll
         for (int l = 0; l < L; ++l) {
-            double x[4], d[4], g[4], t[4], s[4] = {0.0, 0.0, 0.0, 0.0};
+            T x[4], d[4], g[4], t[4], s[4] = {T(0.0), T(0.0), T(0.0), T(0.0)};
             get(kX, l, x); get(kD, l, d); get(kG, l, g);
             point(x, d, step, t);
 #pragma unroll
             for (int c = 0; c < NV; ++c) {
                 s[c] = t[c] - x[c];
-                sl[c] = mul_add(g[c], s[c], sl[c]);
-                largest = max(largest, uint32_t(__double2hiint(s[c])) & 0x7fffffffu);
+                sl[c] = madd<T>(g[c], s[c], sl[c]);
+                largest = max(largest, magnitude_bits(s[c]));
             }
-            const double av = t[3];
-            const double d0 = t[0] - m.mean[l][0], d1 = t[1] - m.mean[l][1], d2 = t[2] - m.mean[l][2];
-            const double* P = m.prec[l];
-            const double v0 = mul_add(P[2], d2, mul_add(P[0], d0, P[1] * d1));
-            const double v1 = mul_add(P[5], d2, mul_add(P[3], d0, P[4] * d1));
-            const double v2 = mul_add(P[8], d2, mul_add(P[6], d0, P[7] * d1));
-            const double D = mul_add(d2, v2, mul_add(d0, v0, d1 * v1));
-            energy = mul_add(av, D, energy);
+            const T av = t[3];
+            const T d0 = t[0] - m.mean[l][0], d1 = t[1] - m.mean[l][1], d2 = t[2] - m.mean[l][2];
+            const T* P = m.prec[l];
+            const T v0 = madd<T>(P[2], d2, madd<T>(P[0], d0, P[1] * d1));
+            const T v1 = madd<T>(P[5], d2, madd<T>(P[3], d0, P[4] * d1));
+            const T v2 = madd<T>(P[8], d2, madd<T>(P[6], d0, P[7] * d1));
+            const T D = madd<T>(d2, v2, madd<T>(d0, v0, d1 * v1));
+            energy = madd<T>(av, D, energy);
             asum += av;
             compose(m, l, t, av, A, pc);
             if (keep) {
 #pragma unroll
                 for (int c = 0; c < NV; ++c) {
-                    ss[c] = mul_add(s[c], s[c], ss[c]);
+                    ss[c] = madd<T>(s[c], s[c], ss[c]);
                     // |s| / (1 + |x|) against the tolerance without the
                     // division, except where rounding could decide.
-                    const double w = 1.0 + fabs(x[c]), as = fabs(s[c]);
-                    if (!(as < tol_lo * w)) moved = moved || as > tol_hi * w || step_reaches(as, w, ctl.inner_tolerance);
+                    const T w = T(1.0) + fabs(x[c]), as = fabs(s[c]);
+                    if constexpr (kFast) moved = moved || !(qdiv(as, w) < T(ctl.inner_tolerance));
+                    else if (!(as < tol_lo * w)) moved = moved || as > tol_hi * w || step_reaches(as, w, ctl.inner_tolerance);
                 }
                 if (best_lost) {
-                    double b[4];
-                    point(x, d, best_at == kBestAtX ? 0.0 : best_step, b);
+                    T b[4];
+                    point(x, d, best_at == kBestAtX ? T(0.0) : best_step, b);
                     store_rec(best_rec(l), b[0], b[1], b[2], b[3]);
                 }
                 store_rec(ring(next, 0, l), s[0], s[1], s[2], s[3]);
@@ -449,9 +503,9 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
                 put(kD, l, pc[0], pc[1], pc[2], A);
             }
         }
-        double res[NV];
+        T res[NV];
 #pragma unroll
-        for (int c = 0; c < NV; ++c) res[c] = c < 3 ? pc[c < 3 ? c : 0] - target(c < 3 ? c : 0) : A - 1.0;
+        for (int c = 0; c < NV; ++c) res[c] = c < 3 ? pc[c < 3 ? c : 0] - target(c < 3 ? c : 0) : A - T(1.0);
         if (keep) {
             small_change = small_change || !moved;
             if (best_here) best_at = kBestAtX;
@@ -462,19 +516,19 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
             store_rec(residual_rec(), res[0], res[1], res[2], res[NV - 1]);
             return;
         }
-        if (!REFINE) energy += 0.01 * asum;
-        double terms[NV], nn[NV];
+        if (!REFINE) energy += T(0.01) * asum;
+        T terms[NV], nn[NV];
 #pragma unroll
         for (int c = 0; c < NV; ++c) {
-            terms[c] = mul_add(0.5 * rho * res[c], res[c], -(lam(c) * res[c]));
+            terms[c] = madd<T>(T(0.5) * rho * res[c], res[c], -(lam(c) * res[c]));
             nn[c] = res[c] * res[c];
         }
-        const double norm = sum(nn), value = energy + sum(terms), slope = sum(sl);
+        const T norm = sum(nn), value = energy + sum(terms), slope = sum(sl);
 
         // A trial that does not move (whose sum of squared motions is zero:
-        // squares below 2^-1074) ends the attempt, unevaluated.
-        if (!at_x && largest < 0x1e600000u) { attempt_failed(); return; }
-        const double tol2 = ctl.outer_tolerance * ctl.outer_tolerance;
+        // squares below the smallest number) ends the attempt, unevaluated.
+        if (!at_x && largest < (kFast ? 0x1a000001u : 0x1e600000u)) { attempt_failed(); return; }
+        const T tol2 = ctl.outer_tolerance * ctl.outer_tolerance;
         const bool feasible = norm < tol2;
         if (isfinite(energy) && isfinite(norm) &&
             (best_at == kNoBest || (feasible && (best_norm() >= tol2 || energy < best_energy())) ||
@@ -497,21 +551,21 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
             state = kLaneGrad;
         } else {
             count(3);
-            if (slope < 0.0 && isfinite(value) && value <= f + 1e-4 * slope) {
+            if (slope < T(0.0) && isfinite(value) && value <= f + T(1e-4) * slope) {
                 if (!counted_grad) { count(0); count(1); ++n_value; ++n_grad; }
-                const double delta = fabs(f - value), size = 0.5 * (fabs(f) + fabs(value));
-                small_change = delta < ctl.inner_tolerance * size;
+                const T delta = fabs(f - value), size = T(0.5) * (fabs(f) + fabs(value));
+                small_change = delta < T(ctl.inner_tolerance) * size;
                 f = value;
                 from_trial = true;
                 state = kLaneGrad;
             } else {
-                step *= 0.5;
+                step *= T(0.5);
                 if (++bt >= 32) attempt_failed();
             }
         }
     }
 
-    __device__ __noinline__ static bool step_reaches(double as, double w, double tol) { return !(as / w < tol); }
+    __device__ __noinline__ static bool step_reaches(T as, T w, T tol) { return !(as / w < tol); }
 
     // The line search ran out of trials: once more from steepest descent,
     // then the end of the inner solve.
@@ -524,65 +578,73 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     // Gradient at the evaluated point (kLaneGrad, after forward()), and the
     // accepted step's curvature pair and termination test.
     __device__ __forceinline__ void backward() {
-        const Models<double>& m = *models_;
+        const Models<T>& m = *models_;
         const bool at_x = !from_trial;
         // Reverse sweep; layer l's slot of d turns from its composite into its gradient.
-        double adj[3], adj3 = REFINE ? 0.0 : rho * res_kept(NV - 1) - lam(NV - 1);
+        T adj[3], adj3 = REFINE ? T(0.0) : rho * res_kept(NV - 1) - lam(NV - 1);
 #pragma unroll
         for (int c = 0; c < 3; ++c) adj[c] = rho * res_kept(c) - lam(c);
 #pragma unroll 1
         for (int l = L - 1; l >= 0; --l) {
-            double t[4], ng[4];
+            T t[4], ng[4];
             get(kX, l, t);
-            const double av = t[3];
+            const T av = t[3];
             {
-                const double d0 = t[0] - m.mean[l][0], d1 = t[1] - m.mean[l][1], d2 = t[2] - m.mean[l][2];
-                const double* P = m.prec[l];
-                const double v0 = mul_add(P[2], d2, mul_add(P[0], d0, P[1] * d1));
-                const double v1 = mul_add(P[5], d2, mul_add(P[3], d0, P[4] * d1));
-                const double v2 = mul_add(P[8], d2, mul_add(P[6], d0, P[7] * d1));
-                const double D = mul_add(d2, v2, mul_add(d0, v0, d1 * v1));
-                const double t0 = mul_add(P[6], d2, mul_add(P[0], d0, P[3] * d1));
-                const double t1 = mul_add(P[7], d2, mul_add(P[1], d0, P[4] * d1));
-                const double t2 = mul_add(P[8], d2, mul_add(P[2], d0, P[5] * d1));
+                const T d0 = t[0] - m.mean[l][0], d1 = t[1] - m.mean[l][1], d2 = t[2] - m.mean[l][2];
+                const T* P = m.prec[l];
+                const T v0 = madd<T>(P[2], d2, madd<T>(P[0], d0, P[1] * d1));
+                const T v1 = madd<T>(P[5], d2, madd<T>(P[3], d0, P[4] * d1));
+                const T v2 = madd<T>(P[8], d2, madd<T>(P[6], d0, P[7] * d1));
+                const T D = madd<T>(d2, v2, madd<T>(d0, v0, d1 * v1));
+                const T t0 = madd<T>(P[6], d2, madd<T>(P[0], d0, P[3] * d1));
+                const T t1 = madd<T>(P[7], d2, madd<T>(P[1], d0, P[4] * d1));
+                const T t2 = madd<T>(P[8], d2, madd<T>(P[2], d0, P[5] * d1));
                 ng[0] = av * (v0 + t0); ng[1] = av * (v1 + t1); ng[2] = av * (v2 + t2);
-                ng[3] = REFINE ? D : D + 0.01;
+                ng[3] = REFINE ? D : D + T(0.01);
             }
             if (l > 0) {
-                double o[4], q[4];
+                T o[4], q[4];
                 get(kD, l, o); get(kD, l - 1, q);
-                const double Al = o[3], dd = q[3], X = m.fX[l], Y = m.fY[l], Z = m.fZ[l];
-                const double n_dd = 1.0 - dd, n_av = 1.0 - av;
-                const double da = mul_add(X, dd, Y * n_dd) - Z * dd;
-                const double db = mul_add(Z, n_av, X * av - Y * av);
-                const double ya = Y * av * n_dd, yd = Y * n_dd, zd = Z * dd, zdn = zd * n_av, zn = Z * n_av, ad = av * dd;
-                const bool big = Al > 1e-12;
-                double fv[3], fs[3], fd[3], ga[3], gp[3];
-                blend_all3(m.mode[l], t, q, fv, fs, fd);
-                const double y = reciprocal(Al);
+                const T Al = o[3], dd = q[3], X = m.fX[l], Y = m.fY[l], Z = m.fZ[l];
+                const T n_dd = T(1.0) - dd, n_av = T(1.0) - av;
+                const T da = madd<T>(X, dd, Y * n_dd) - Z * dd;
+                const T db = madd<T>(Z, n_av, X * av - Y * av);
+                const T ya = Y * av * n_dd, yd = Y * n_dd, zd = Z * dd, zdn = zd * n_av, zn = Z * n_av, ad = av * dd;
+                const bool big = Al > T(1e-12);
+                T fv[3], fs[3], fd[3], ga[3], gp[3];
+                blend_all(m, l, t, q, fv, fs, fd);
+                T y;   // (FP32: times the approximate reciprocal)
+                if constexpr (kFast) y = big ? qdiv(T(1), Al) : T(1); else y = reciprocal(Al);
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
-                    const double v = adj[c], s = t[c], cc = q[c];
-                    const double ds = mul_add(ad, fs[c], ya);
-                    const double dc = mul_add(ad, fd[c], zdn);
-                    const double pa = mul_add(fv[c], dd, yd * s) - zd * cc;
-                    const double pd = mul_add(zn, cc, fv[c] * av - Y * av * s);
-                    const double na = pa - o[c] * da, np = pd - o[c] * db;
-                    const double qa = quotient(na, Al, y), qp = quotient(np, Al, y), qs = quotient(ds, Al, y),
-                                 qc = quotient(dc, Al, y);
-                    ga[c] = v * (big ? qa : pa);
-                    gp[c] = v * (big ? qp : pd);
-                    ng[c] += v * (big ? qs : ds);
-                    adj[c] = v * (big ? qc : dc);
+                    const T v = adj[c], s = t[c], cc = q[c];
+                    const T ds = madd<T>(ad, fs[c], ya);
+                    const T dc = madd<T>(ad, fd[c], zdn);
+                    const T pa = madd<T>(fv[c], dd, yd * s) - zd * cc;
+                    const T pd = madd<T>(zn, cc, fv[c] * av - Y * av * s);
+                    if constexpr (kFast) {
+                        ga[c] = v * (big ? madd<T>(-o[c], da, pa) * y : pa);
+                        gp[c] = v * (big ? madd<T>(-o[c], db, pd) * y : pd);
+                        ng[c] += v * (big ? ds * y : ds);
+                        adj[c] = v * (big ? dc * y : dc);
+                    } else {
+                        const T na = pa - o[c] * da, np = pd - o[c] * db;
+                        const T qa = quotient(na, Al, y), qp = quotient(np, Al, y), qs = quotient(ds, Al, y),
+                                qc = quotient(dc, Al, y);
+                        ga[c] = v * (big ? qa : pa);
+                        gp[c] = v * (big ? qp : pd);
+                        ng[c] += v * (big ? qs : ds);
+                        adj[c] = v * (big ? qc : dc);
+                    }
                 }
                 if constexpr (REFINE) {
-                    double ta = adj3 * da, tp = adj3 * db;
+                    T ta = adj3 * da, tp = adj3 * db;
                     ta += ga[0]; ta += ga[1]; ta += ga[2];
                     tp += gp[0]; tp += gp[1]; tp += gp[2];
                     ng[3] += ta;
                     adj3 = tp;
                 } else {
-                    const double g3 = adj3 * da, p3 = adj3 * db;
+                    const T g3 = adj3 * da, p3 = adj3 * db;
                     ng[3] += (ga[0] + ga[1]) + (ga[2] + g3);
                     adj3 = (gp[0] + gp[1]) + (gp[2] + p3);
                 }
@@ -596,35 +658,35 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         if (at_x) {
 #pragma unroll
             for (int l = 0; l < L; ++l) {
-                double ng[4];
+                T ng[4];
                 get(kD, l, ng);
                 put(kG, l, ng[0], ng[1], ng[2], ng[3]);
             }
             state = kLaneDir;
             return;
         }
-        double sy[NV], yy[NV], ya = 0.0;
+        T sy[NV], yy[NV], ya = T(0.0);
 #pragma unroll
-        for (int c = 0; c < NV; ++c) { sy[c] = 0.0; yy[c] = 0.0; }
-        double step_taken[L][4];
+        for (int c = 0; c < NV; ++c) { sy[c] = T(0.0); yy[c] = T(0.0); }
+        T step_taken[L][4];
 #pragma unroll
         for (int l = 0; l < L; ++l) load_rec(ring(next, 0, l), step_taken[l]);
 #pragma unroll
         for (int l = 0; l < L; ++l) {
-            double ng[4], g[4], yv[4] = {0.0, 0.0, 0.0, 0.0};
-            const double* s = step_taken[l];
+            T ng[4], g[4], yv[4] = {T(0.0), T(0.0), T(0.0), T(0.0)};
+            const T* s = step_taken[l];
             get(kD, l, ng); get(kG, l, g);
 #pragma unroll
             for (int c = 0; c < NV; ++c) {
                 yv[c] = ng[c] - g[c];
-                sy[c] = mul_add(s[c], yv[c], sy[c]);
-                yy[c] = mul_add(yv[c], yv[c], yy[c]);
+                sy[c] = madd<T>(s[c], yv[c], sy[c]);
+                yy[c] = madd<T>(yv[c], yv[c], yy[c]);
             }
-            if (REFINE) { const double dy = ng[3] - g[3]; ya = mul_add(dy, dy, ya); }
+            if (REFINE) { const T dy = ng[3] - g[3]; ya = madd<T>(dy, dy, ya); }
             store_rec(ring(next, 1, l), yv[0], yv[1], yv[2], yv[3]);
             put(kG, l, ng[0], ng[1], ng[2], ng[3]);
         }
-        double yyt = sum(yy);
+        T yyt = sum(yy);
         if (REFINE) yyt += ya;
         if (curvature(sum(sy), ss_kept(), yyt)) {
             next = next + 1 == kLaneRing ? 0 : next + 1;
@@ -635,16 +697,20 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         else state = kLaneDir;
     }
 
+    __device__ __forceinline__ static T inverse(T v) {
+        if constexpr (kFast) return qdiv(T(1), v); else return __drcp_rn(v);
+    }
     // sy > 1e-9 sqrt(ss yy), sy > 0 and 1 / sy finite: by squares, except
     // where rounding, under- or overflow could decide.
-    __device__ __forceinline__ static bool curvature(double sy, double ss, double yy) {
-        if (!(sy > 0.0)) return false;
-        const double t = 1e-18 * (ss * yy), r = sy * sy;
+    __device__ __forceinline__ static bool curvature(T sy, T ss, T yy) {
+        if constexpr (kFast) return sy > T(0) && sy * sy > T(1e-18) * (ss * yy) && isfinite(qdiv(T(1), sy));
+        if (!(sy > T(0.0))) return false;
+        const T t = T(1e-18) * (ss * yy), r = sy * sy;
         if (t > 1e-250 && t < 1e250 && r < 1e250 && fabs(r - t) > 1e-12 * t) return r > t;
         return curvature_exact(sy, ss, yy);
     }
-    __device__ __noinline__ static bool curvature_exact(double sy, double ss, double yy) {
-        return sy > 1e-9 * sqrt(ss * yy) && sy > 0.0 && isfinite(1.0 / sy);
+    __device__ __noinline__ static bool curvature_exact(T sy, T ss, T yy) {
+        return sy > T(1e-9) * sqrt(ss * yy) && sy > T(0.0) && isfinite(T(1.0) / sy);
     }
 
     // ---------------------------------------------------------- direction --
@@ -659,83 +725,83 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         if (what == kReset) { valid = 0; next = 0; }
         second = steep;
         bt = 0;
-        step = 1.0;
+        step = T(1.0);
         state = kLaneTrial;
     }
 
     // Forms d from x, g and the ring (static: it touches none of the pixel's
     // other state).
     enum : int { kStationary = 0, kFormed = 1, kReset = 2 };
-    __device__ __forceinline__ static int form_direction(double* base, int valid, int next, bool steep, bool opaque,
+    __device__ __forceinline__ static int form_direction(T* base, int valid, int next, bool steep, bool opaque,
                                                       bool smooth, bool finite_f) {
         uint32_t freem = 0;
         {
-            double pg[NV];
+            T pg[NV];
 #pragma unroll
-            for (int c = 0; c < NV; ++c) pg[c] = 0.0;
+            for (int c = 0; c < NV; ++c) pg[c] = T(0.0);
 #pragma unroll 1
             for (int l = 0; l < L; ++l) {
-                double x[4], g[4], v[4];
+                T x[4], g[4], v[4];
                 get(kX, l, x); get(kG, l, g);
-                v[3] = 0.0;
+                v[3] = T(0.0);
 #pragma unroll
                 for (int c = 0; c < NV; ++c) {
                     const bool fr = !fixed_at(opaque, smooth, l, c, x[c], g[c]);
                     freem |= fr ? 1u << (l * 4 + c) : 0u;
-                    v[c] = fr ? g[c] : 0.0;
-                    pg[c] = mul_add(v[c], v[c], pg[c]);
+                    v[c] = fr ? g[c] : T(0.0);
+                    pg[c] = madd<T>(v[c], v[c], pg[c]);
                 }
                 put(kD, l, v[0], v[1], v[2], v[3]);
             }
-            if (!steep && (sum(pg) < 1e-16 || !finite_f)) return kStationary;
+            if (!steep && (sum(pg) < T(1e-16) || !finite_f)) return kStationary;
         }
-        double q[L][4];
+        T q[L][4];
 #pragma unroll
         for (int l = 0; l < L; ++l) get(kD, l, q[l]);
         // The pairs' components outside the free set are read as zeros (a
         // select each; skipping their operations instead takes a branch each,
         // and the kernel 1.1 times as long). q is zero there throughout, so
         // its own products need no select.
-        double scaling = 1.0;
+        T scaling = T(1.0);
         bool have_scaling = false;
-        double2* coeff = slot(4 * L);
+        double2* coeff = slot(2 * L * kUnits);   // (one pair a unit)
 #pragma unroll 1
         for (int j = 0; j < valid; ++j) {
             int k = next - 1 - j;
             k = k < 0 ? k + kLaneRing : k;
-            double dot[NV], sy[NV], ss[NV], yy[NV];
+            T dot[NV], sy[NV], ss[NV], yy[NV];
 #pragma unroll
-            for (int c = 0; c < NV; ++c) { dot[c] = 0.0; sy[c] = 0.0; ss[c] = 0.0; yy[c] = 0.0; }
-            double ym[L][4];
+            for (int c = 0; c < NV; ++c) { dot[c] = T(0.0); sy[c] = T(0.0); ss[c] = T(0.0); yy[c] = T(0.0); }
+            T ym[L][4];
 #pragma unroll
             for (int l = 0; l < L; ++l) load_rec(ring(base, k, 1, l), ym[l]);
 #pragma unroll
             for (int l = 0; l < L; ++l) {
-                double sv[4];
-                double* yv = ym[l];
+                T sv[4];
+                T* yv = ym[l];
                 load_rec(ring(base, k, 0, l), sv);
 #pragma unroll
                 for (int c = 0; c < NV; ++c) {
                     const bool fr = freem >> (l * 4 + c) & 1u;
-                    const double s1 = fr ? sv[c] : 0.0, y1 = fr ? yv[c] : 0.0;
+                    const T s1 = fr ? sv[c] : T(0.0), y1 = fr ? yv[c] : T(0.0);
                     yv[c] = y1;
-                    dot[c] = mul_add(s1, q[l][c], dot[c]);
-                    sy[c] = mul_add(s1, y1, sy[c]);
-                    ss[c] = mul_add(s1, s1, ss[c]);
-                    yy[c] = mul_add(y1, y1, yy[c]);
+                    dot[c] = madd<T>(s1, q[l][c], dot[c]);
+                    sy[c] = madd<T>(s1, y1, sy[c]);
+                    ss[c] = madd<T>(s1, s1, ss[c]);
+                    yy[c] = madd<T>(y1, y1, yy[c]);
                 }
             }
-            const double syt = sum(sy), yyt = sum(yy);
-            const double inv = curvature(syt, sum(ss), yyt) ? __drcp_rn(syt) : 0.0;
-            const double co = sum(dot) * inv;
+            const T syt = sum(sy), yyt = sum(yy);
+            const T inv = curvature(syt, sum(ss), yyt) ? inverse(syt) : T(0.0);
+            const T co = sum(dot) * inv;
 #pragma unroll
             for (int l = 0; l < L; ++l)
 #pragma unroll
-                for (int c = 0; c < NV; ++c) q[l][c] = mul_add(-co, ym[l][c], q[l][c]);
-            if (!have_scaling && inv > 0.0 && yyt > 0.0) { scaling = syt / yyt; have_scaling = true; }
-            coeff[j * kLaneBlock] = make_double2(co, inv);
+                for (int c = 0; c < NV; ++c) q[l][c] = madd<T>(-co, ym[l][c], q[l][c]);
+            if (!have_scaling && inv > T(0.0) && yyt > T(0.0)) { scaling = qdiv(syt, yyt); have_scaling = true; }
+            coeff[j * kLaneBlock] = make_double2(co, inv);   // (exact in FP32 too)
         }
-        scaling = fmax(1e-12, fmin(1e3, scaling));
+        scaling = fmax(T(1e-12), fmin(T(1e3), scaling));
 #pragma unroll
         for (int l = 0; l < L; ++l)
 #pragma unroll
@@ -744,50 +810,50 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         for (int j = valid - 1; j >= 0; --j) {
             int k = next - 1 - j;
             k = k < 0 ? k + kLaneRing : k;
-            double dot[NV], sv[L][4];
+            T dot[NV], sv[L][4];
 #pragma unroll
-            for (int c = 0; c < NV; ++c) dot[c] = 0.0;
+            for (int c = 0; c < NV; ++c) dot[c] = T(0.0);
 #pragma unroll
             for (int l = 0; l < L; ++l) {
-                double yv[4];
+                T yv[4];
                 load_rec(ring(base, k, 1, l), yv); load_rec(ring(base, k, 0, l), sv[l]);
 #pragma unroll
-                for (int c = 0; c < NV; ++c) dot[c] = mul_add(yv[c], q[l][c], dot[c]);
+                for (int c = 0; c < NV; ++c) dot[c] = madd<T>(yv[c], q[l][c], dot[c]);
             }
             const double2 ci = coeff[j * kLaneBlock];
-            const double w = mul_add(-sum(dot), ci.y, ci.x);
+            const T w = madd<T>(-sum(dot), T(ci.y), T(ci.x));
 #pragma unroll
             for (int l = 0; l < L; ++l)
 #pragma unroll
                 for (int c = 0; c < NV; ++c)
-                    q[l][c] = mul_add(w, freem >> (l * 4 + c) & 1u ? sv[l][c] : 0.0, q[l][c]);
+                    q[l][c] = madd<T>(w, freem >> (l * 4 + c) & 1u ? sv[l][c] : T(0.0), q[l][c]);
         }
 #pragma unroll
         for (int l = 0; l < L; ++l) put(kD, l, q[l][0], q[l][1], q[l][2], q[l][3]);
-        double descent[NV];
+        T descent[NV];
 #pragma unroll
-        for (int c = 0; c < NV; ++c) descent[c] = 0.0;
+        for (int c = 0; c < NV; ++c) descent[c] = T(0.0);
 #pragma unroll 1
         for (int l = 0; l < L; ++l) {
-            double x[4], g[4], d[4];
+            T x[4], g[4], d[4];
             get(kX, l, x); get(kG, l, g); get(kD, l, d);
 #pragma unroll
             for (int c = 0; c < NV; ++c) {
-                double v = -d[c];
-                if (fixed_bounds(opaque, smooth, l, c) || (x[c] <= 0.0 && v < 0.0) || (x[c] >= 1.0 && v > 0.0)) v = 0.0;
+                T v = -d[c];
+                if (fixed_bounds(opaque, smooth, l, c) || (x[c] <= T(0.0) && v < T(0.0)) || (x[c] >= T(1.0) && v > T(0.0))) v = T(0.0);
                 d[c] = v;
-                descent[c] = mul_add(v, g[c], descent[c]);
+                descent[c] = madd<T>(v, g[c], descent[c]);
             }
             put(kD, l, d[0], d[1], d[2], d[3]);
         }
-        if (!steep && !(sum(descent) < 0.0)) {
+        if (!steep && !(sum(descent) < T(0.0))) {
 #pragma unroll 1
             for (int l = 0; l < L; ++l) {
-                double x[4], g[4], d[4];
+                T x[4], g[4], d[4];
                 get(kX, l, x); get(kG, l, g);
-                d[3] = 0.0;
+                d[3] = T(0.0);
 #pragma unroll
-                for (int c = 0; c < NV; ++c) d[c] = fixed_at(opaque, smooth, l, c, x[c], g[c]) ? 0.0 : -g[c];
+                for (int c = 0; c < NV; ++c) d[c] = fixed_at(opaque, smooth, l, c, x[c], g[c]) ? T(0.0) : -g[c];
                 put(kD, l, d[0], d[1], d[2], d[3]);
             }
             return kReset;
@@ -799,34 +865,36 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     // End of an outer step (kLaneEnd): multipliers, penalty, and the next
     // outer step, the next start, or the pixel's result.
     enum : int { kNextOuter, kNextStart, kFinished };
-    __device__ __forceinline__ int end_outer(Outer& o) {
-        double r[4], ox[L][4], nn[NV], mo[NV];
+    __device__ __forceinline__ int end_outer(Outer& o, bool& capped) {
+        T r[4], ox[L][4], nn[NV], mo[NV];
         o = load_outer();
         load_rec(residual_rec(), r);
 #pragma unroll
         for (int l = 0; l < L; ++l) load_rec(ox_rec(l), ox[l]);
-        const double tol2 = ctl.outer_tolerance * ctl.outer_tolerance;
+        const T tol2 = ctl.outer_tolerance * ctl.outer_tolerance;
 #pragma unroll
-        for (int c = 0; c < NV; ++c) { nn[c] = r[c] * r[c]; mo[c] = 0.0; }
-        const double norm = sum(nn);
+        for (int c = 0; c < NV; ++c) { nn[c] = r[c] * r[c]; mo[c] = T(0.0); }
+        const T norm = sum(nn);
         const bool feasible = norm < tol2;
 #pragma unroll
-        for (int c = 0; c < NV; ++c) lam(c) = mul_add(-rho, r[c], lam(c));
-        if (norm > 0.0625 * o.oldnorm) rho *= 10.0;
+        for (int c = 0; c < NV; ++c) lam(c) = madd<T>(-rho, r[c], lam(c));
+        if (norm > T(0.0625) * o.oldnorm) rho *= T(10.0);
 #pragma unroll
         for (int l = 0; l < L; ++l) {
-            double x[4];
+            T x[4];
             get(kX, l, x);
 #pragma unroll
-            for (int c = 0; c < NV; ++c) { const double dl = x[c] - ox[l][c]; mo[c] = mul_add(dl, dl, mo[c]); }
+            for (int c = 0; c < NV; ++c) { const T dl = x[c] - ox[l][c]; mo[c] = madd<T>(dl, dl, mo[c]); }
         }
-        const double motion = sum(mo);
-        o.frozen = (motion == 0.0 && !best_moved) ? o.frozen + 1 : 0;
+        const T motion = sum(mo);
+        o.frozen = (motion == T(0.0) && !best_moved) ? o.frozen + 1 : 0;
         int what = kFinished;
         if (!(ctl.frozen_stop > 0 && o.frozen >= ctl.frozen_stop) && !(motion < tol2 && feasible) &&
             o.outer + 1 < ctl.outer) {
             ++o.outer;
             what = kNextOuter;
+        } else if (kFast && ctl.cap_is_miss && !(motion < tol2 && feasible)) {
+            capped = true;   // the FP64 re-solve gives the pixel the method's own result
         } else if (o.start + 1 < ctl.starts) {
             ++o.start;
             what = kNextStart;
@@ -840,13 +908,13 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
         count(4);
 #pragma unroll
         for (int l = 0; l < L; ++l) {
-            double x[4];
+            T x[4];
             get(kX, l, x);
             store_rec(ox_rec(l), x[0], x[1], x[2], x[3]);
-            put(kD, l, 0.0, 0.0, 0.0, 0.0);
+            put(kD, l, T(0.0), T(0.0), T(0.0), T(0.0));
         }
         best_moved = false;
-        step = 0.0;
+        step = T(0.0);
         state = kLaneOuter;
     }
 
@@ -864,39 +932,40 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     }
 
     // The start-0 seed of component c of layer l.
-    __device__ __forceinline__ double seed(const Outer& o, int l, int c) const {
+    __device__ __forceinline__ T seed(const Outer& o, int l, int c) const {
         const size_t i = size_t(o.pixel);
         if constexpr (REFINE) {
-            if (c == 3) return pinned_alpha(o, l);
-            return (a.smooth && l == 0) ? background(o, c) : a.first[(size_t(l) * size_t(a.n) + i) * 4 + c];
+            if (c == 3) return T(pinned_alpha(o, l));
+            return T((a.smooth && l == 0) ? background(o, c) : a.first[(size_t(l) * size_t(a.n) + i) * 4 + c]);
         } else {
             const float* wp;
             if constexpr (BATCH) wp = a.jobs[o.job].warm; else wp = a.warm;
-            if (wp) return double(wp[i * size_t(4 * L) + (c == 3 ? l : L + 3 * l + c)]);
-            if (c == 3) return (a.opaque && l == 0) ? 1.0 : 0.5;
-            return fmin(1.0, fmax(0.0, models_->mean[l][c]));
+            if (wp) return T(wp[i * size_t(4 * L) + (c == 3 ? l : L + 3 * l + c)]);
+            if (c == 3) return (a.opaque && l == 0) ? T(1.0) : T(0.5);
+            return fmin(T(1.0), fmax(T(0.0), models_->mean[l][c]));
         }
     }
 
     // Bounds of component c of layer l applied to v.
-    __device__ __forceinline__ double clamp_bounds(const Outer& o, int l, int c, double v) const {
+    __device__ __forceinline__ T clamp_bounds(const Outer& o, int l, int c, T v) const {
         if (REFINE && c == 3) return v;
-        double lo = 0.0, hi = 1.0;
-        if (l == 0 && c == 3 && a.opaque) lo = 1.0;
-        if (REFINE && l == 0 && c != 3 && a.smooth) lo = hi = background(o, c);
+        T lo = T(0.0), hi = T(1.0);
+        if (l == 0 && c == 3 && a.opaque) lo = T(1.0);
+        if (REFINE && l == 0 && c != 3 && a.smooth) lo = hi = T(background(o, c));
         return v < lo ? lo : (v > hi ? hi : v);
     }
 
     // Component c of layer l of x in shared memory.
-    __device__ __forceinline__ static double* x_at(int l, int c) {
-        return reinterpret_cast<double*>(slot(kX * 2 * L + 2 * l + (c >> 1))) + (c & 1);
+    __device__ __forceinline__ static T* x_at(int l, int c) {
+        if constexpr (kFast) return reinterpret_cast<T*>(slot(l)) + c;
+        else return reinterpret_cast<T*>(slot(2 * l + (c >> 1))) + (c & 1);
     }
 
     // Starting point o.start: the seeds, all loads in flight at once; the
     // further starts one component at a time (rare).
     __device__ __forceinline__ void begin_start(Outer& o) {
         if (o.start == 0) {
-            double v[L][4];
+            T v[L][4];
 #pragma unroll
             for (int l = 0; l < L; ++l)
 #pragma unroll
@@ -912,41 +981,41 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
             further_start(o);
         }
 #pragma unroll
-        for (int c = 0; c < NV; ++c) lam(c) = 0.0;
-        rho = 100.0;
+        for (int c = 0; c < NV; ++c) lam(c) = T(0.0);
+        rho = T(100.0);
         o.outer = 0;
         o.frozen = 0;
     }
 
     __device__ __forceinline__ void further_start(const Outer& o) const {
-        const Models<double>& m = *models_;
+        const Models<T>& m = *models_;
         const int s = o.start;
 #pragma unroll 1
         for (int k = 0; k < 4 * L; ++k) {
             const int l = k >> 2, c = k & 3;
-            double v;
-            if (c == 3) v = REFINE ? pinned_alpha(o, l) : (s == 1 ? (l == 0 ? 1.0 : 0.0) : 0.5);
-            else if (s == 2) v = fmax(0.05, fmin(0.95, m.mean[l][c]));
-            else v = (!REFINE && l == 0) ? fmin(1.0, fmax(0.0, image(o)[3 * size_t(o.pixel) + c])) : m.mean[l][c];
+            T v;
+            if (c == 3) v = REFINE ? T(pinned_alpha(o, l)) : (s == 1 ? (l == 0 ? T(1.0) : T(0.0)) : T(0.5));
+            else if (s == 2) v = fmax(T(0.05), fmin(T(0.95), m.mean[l][c]));
+            else v = (!REFINE && l == 0) ? fmin(T(1.0), fmax(T(0.0), T(image(o)[3 * size_t(o.pixel) + c]))) : m.mean[l][c];
             *x_at(l, c) = clamp_bounds(o, l, c, v);
         }
         if (s != 2) return;
         // Move Dodge/Burn sources into the unsaturated branch.
 #pragma unroll 1
         for (int c = 0; c < 3; ++c) {
-            double da = *x_at(0, 3), dest = *x_at(0, c);
+            T da = *x_at(0, 3), dest = *x_at(0, c);
 #pragma unroll 1
             for (int l = 1; l < L; ++l) {
-                const double al = *x_at(l, 3), X = m.fX[l], Y = m.fY[l], Z = m.fZ[l];
-                const double Al = X * al * da + Y * al * (1.0 - da) + Z * da * (1.0 - al);
-                double sv = *x_at(l, c);
-                if (dest >= 0.0 && dest <= 1.0 && m.mode[l] == 6) sv = fmin(sv, fmax(0.0, 1.0 - dest - 0.05));
-                if (dest >= 0.0 && dest <= 1.0 && m.mode[l] == 7) sv = fmax(sv, fmin(1.0, 1.0 - dest + 0.05));
+                const T al = *x_at(l, 3), X = m.fX[l], Y = m.fY[l], Z = m.fZ[l];
+                const T Al = X * al * da + Y * al * (T(1.0) - da) + Z * da * (T(1.0) - al);
+                T sv = *x_at(l, c);
+                if (dest >= T(0.0) && dest <= T(1.0) && m.mode[l] == 6) sv = fmin(sv, fmax(T(0.0), T(1.0) - dest - T(0.05)));
+                if (dest >= T(0.0) && dest <= T(1.0) && m.mode[l] == 7) sv = fmax(sv, fmin(T(1.0), T(1.0) - dest + T(0.05)));
                 sv = clamp_bounds(o, l, c, sv);
                 *x_at(l, c) = sv;
-                const double pre = blend_value_call<double>(m.mode[l], sv, dest) * al * da +
-                                   Y * al * (1.0 - da) * sv + Z * da * (1.0 - al) * dest;
-                dest = Al > 1e-12 ? pre / Al : pre;
+                const T pre = blend_value_call<T>(m.mode[l], sv, dest) * al * da +
+                                   Y * al * (T(1.0) - da) * sv + Z * da * (T(1.0) - al) * dest;
+                dest = Al > T(1e-12) ? pre / Al : pre;
                 da = Al;
             }
         }
@@ -957,27 +1026,30 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     // list. The point written is the best point, whose constraint norm is
     // best_norm (the same operations on the same values as a check of the
     // written point); a pixel without one writes its seed, checked here.
-    __device__ __forceinline__ void store(const Outer& o, bool skipped) {
+    __device__ __forceinline__ void store(const Outer& o, bool skipped, bool capped) {
         const size_t n = pixels(o), i = size_t(o.pixel);
         double* outp;
         int32_t* stp;
         if constexpr (BATCH) { outp = a.jobs[o.job].out; stp = a.jobs[o.job].status; }
         else { outp = a.out; stp = a.status; }
+        T w[L][4];
         double v[L][4];
         if (best_at == kBestStored) {
 #pragma unroll
-            for (int l = 0; l < L; ++l) load_rec(best_rec(l), v[l]);
+            for (int l = 0; l < L; ++l) load_rec(best_rec(l), w[l]);
         } else if (best_at == kBestAtX) {
 #pragma unroll
-            for (int l = 0; l < L; ++l) get(kX, l, v[l]);
+            for (int l = 0; l < L; ++l) get(kX, l, w[l]);
         } else {
 #pragma unroll
             for (int l = 0; l < L; ++l)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) v[l][c] = seed(o, l, c);
+                for (int c = 0; c < 4; ++c) w[l][c] = seed(o, l, c);
         }
 #pragma unroll
         for (int l = 0; l < L; ++l) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) v[l][c] = double(w[l][c]);
             if (REFINE) v[l][3] = pinned_alpha(o, l);
             else if (l == 0 && a.opaque) v[l][3] = 1.0;
             if (REFINE && l == 0 && a.smooth)
@@ -993,14 +1065,16 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
             if (a.input_failed) atomicAdd(a.input_failed, 1);
             return;
         }
-        if (best_at == kNoBest) best_norm() = written_norm(*models_, outp, image(o) + 3 * i, n, i);
-        const bool miss = !(best_norm() < ctl.outer_tolerance * ctl.outer_tolerance);
+        // FP64: the written best point's norm is best_norm, the same operations
+        // on the same values. FP32, and a pixel without a best point: checked.
+        const double norm = kFast || best_at == kNoBest ? written_norm(*models_, outp, image(o) + 3 * i, n, i) : double(best_norm());
+        const bool miss = capped || !(norm < ctl.outer_tolerance * ctl.outer_tolerance);
         if (stp) stp[i] = miss ? 3 : 0;
         if (miss && a.miss_list) a.miss_list[atomicAdd(a.miss_count, 1)] = int32_t(o.gidx);
     }
 
     // Constraint norm of the written point, one channel at a time.
-    __device__ __noinline__ static double written_norm(const Models<double>& m, const double* outp, const double* rgb,
+    __device__ __noinline__ static double written_norm(const Models<T>& m, const double* outp, const double* rgb,
                                                        size_t n, size_t i) {
         double total = 0.0, A = 0.0, first_two = 0.0;
 #pragma unroll 1
@@ -1040,20 +1114,20 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
                 if (a.jobs[mid].offset <= int64_t(o.gidx)) lo = mid; else hi = mid - 1;
             }
             o.job = lo;
-            models_ = static_cast<const Models<double>*>(a.models) + a.jobs[lo].model;
+            models_ = static_cast<const Models<T>*>(a.models) + a.jobs[lo].model;
             o.pixel = o.gidx - int(a.jobs[lo].offset);
         }
         const size_t i = size_t(o.pixel);
         const double* p = image(o) + 3 * i;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) target(c) = p[c];
+        for (int c = 0; c < 3; ++c) target(c) = T(p[c]);
         best_at = kNoBest;
         best_norm() = INFINITY; best_energy() = INFINITY;
         if (a.counters)
 #pragma unroll
             for (int k = 0; k < 5; ++k) a.counters[5 * size_t(o.gidx) + k] = 0;
         o.start = 0;
-        o.oldnorm = 0.0;
+        o.oldnorm = T(0.0);
         return !(REFINE && a.input_status && a.input_status[i] != 0);
     }
 
@@ -1088,16 +1162,16 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
             if (live == 0) break;
             if (ne > 0 && (8 * ne >= kOuterQuorum * live || nf == 0)) {
                 int what = kFinished;
-                bool write = false, skipped = false;
+                bool write = false, skipped = false, capped = false;
                 Outer o{};
                 if (state == kLaneEnd) {
-                    what = end_outer(o);
+                    what = end_outer(o, capped);
                     write = what == kFinished;
                 }
                 // Finished pixels are written, and the lanes without a pixel
                 // take the next queue entries together.
                 for (;;) {
-                    if (write) { store(o, skipped); write = false; state = kLaneFetch; }
+                    if (write) { store(o, skipped, capped); write = false; capped = false; state = kLaneFetch; }
                     const unsigned want = __ballot_sync(full, state == kLaneFetch);
                     if (want == 0) break;
                     const int leader = __ffs(want) - 1;
@@ -1148,11 +1222,11 @@ template <int L, bool REFINE, bool BATCH> struct LaneSolver {
     }
 };
 
-template <int L, bool REFINE, bool BATCH>
-__global__ void __launch_bounds__(kLaneBlock, lane_blocks_per_sm(L))
-solve_lanes(const __grid_constant__ Models<double> m, const __grid_constant__ SolverControls ctl,
+template <class T, int L, bool REFINE, bool BATCH>
+__global__ void __launch_bounds__(kLaneBlock, lane_blocks_per_sm(L, sizeof(T) == 4))
+solve_lanes(const __grid_constant__ Models<T> m, const __grid_constant__ SolverControls ctl,
             const __grid_constant__ SolveArgs a) {
-    LaneSolver<L, REFINE, BATCH> solver(&m, ctl, a);
+    LaneSolver<T, L, REFINE, BATCH> solver(&m, ctl, a);
     solver.run();
 }
 

@@ -26,7 +26,7 @@ namespace unb {
 // variant 7: the refinement of 6 with its cold values in the global array,
 // capped for 4 blocks per SM (first passes run 3).
 constexpr int kFp32Variants = 6, kFp64Variants = 8;
-constexpr int kFp64Lanes = kFp64Variants;   // one pixel per lane (lane_solver.cuh)
+constexpr int kFp64Lanes = kFp64Variants, kFp32Lanes = kFp32Variants;   // one pixel per lane (lane_solver.cuh)
 inline bool variant_global_history(bool fp64, int variant) { return fp64 ? variant >= 2 : variant == 4; }
 // FP64 variants whose kernels can defer and resume pixels (SolveArgs::
 // defer_outer / resume): the refinement's variant 7. (Deferral was measured
@@ -64,6 +64,8 @@ template <int L> cudaError_t solve_batch_fp64_layers(int variant, const SolverCo
 // Lane kernels (lane_l<L>.cu).
 template <int L> cudaError_t solve_lanes_layers(bool refine, bool batch, const Models<double>& m,
                                                 const SolverControls& c, const SolveArgs& a, int sms, cudaStream_t s);
+template <int L> cudaError_t solve_lanes_fp32_layers(bool refine, const Models<float>& m, const SolverControls& c,
+                                                     const SolveArgs& a, int sms, cudaStream_t s);
 #define UNB_DECLARE_LAYER_SOLVES(L)                                                                              \
     template <> cudaError_t solve_fp32_layers<L>(bool, int, const Models<float>&, const SolverControls&,         \
                                                  const SolveArgs&, int, int, cudaStream_t);                      \
@@ -74,7 +76,9 @@ template <int L> cudaError_t solve_lanes_layers(bool refine, bool batch, const M
     template <> cudaError_t solve_batch_fp64_layers<L>(int, const SolverControls&, const SolveArgs&, int, int,   \
                                                        cudaStream_t);                                            \
     template <> cudaError_t solve_lanes_layers<L>(bool, bool, const Models<double>&, const SolverControls&,      \
-                                                  const SolveArgs&, int, cudaStream_t);
+                                                  const SolveArgs&, int, cudaStream_t);                          \
+    template <> cudaError_t solve_lanes_fp32_layers<L>(bool, const Models<float>&, const SolverControls&,        \
+                                                       const SolveArgs&, int, cudaStream_t);
 UNB_DECLARE_LAYER_SOLVES(1)
 UNB_DECLARE_LAYER_SOLVES(2)
 UNB_DECLARE_LAYER_SOLVES(3)

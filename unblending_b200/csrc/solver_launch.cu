@@ -22,6 +22,8 @@ template <class F> cudaError_t by_layers(int L, F&& f) {
 
 cudaError_t launch_solve_fp32(int L, bool refine, int variant, const Models<float>& m, const SolverControls& c,
                               const SolveArgs& a, int threads, int sms, cudaStream_t s) {
+    if (variant == kFp32Lanes)
+        return by_layers(L, [&](auto k) { return solve_lanes_fp32_layers<decltype(k)::value>(refine, m, c, a, sms, s); });
     return by_layers(L, [&](auto k) { return solve_fp32_layers<decltype(k)::value>(refine, variant, m, c, a, threads, sms, s); });
 }
 

@@ -478,9 +478,9 @@ void attach_history(SolveArgs& a, void* array, bool fp64, int variant, int sms) 
     a.history_lanes = int(history_lanes(sms));
 }
 // The same for the lane kernels (`array` of lane_history_bytes(L, sms) bytes).
-void attach_lane_history(SolveArgs& a, void* array, int L, int sms) {
+void attach_lane_history(SolveArgs& a, void* array, int L, int sms, bool fp32 = false) {
     a.history = array;
-    a.history_lanes = lane_blocks(L, sms) * kLaneBlock;
+    a.history_lanes = lane_blocks(L, sms, fp32) * kLaneBlock;
 }
 
 SolverControls controls(const unblending_solver_options& so) {
@@ -687,8 +687,11 @@ PassResult enqueue_pass(Context& c, const Spec& sp, bool refine, const unblendin
     const bool lanes = lane_solve(so);
     const int v64 = lanes ? kFp64Lanes : fp64_variant(so, refine);
     // (the FP32 solve's global history, where its variant has one, is of the quads' size)
-    const size_t quad_history = lanes && so.precision == UNBLENDING_PRECISION_FP64 ? 0 : history_bytes(L, sizeof(double), c.sms);
-    void* history = c.history.get<unsigned char>(std::max(quad_history, lanes ? lane_history_bytes(L, c.sms) : 0));
+    const bool fp32 = so.precision == UNBLENDING_PRECISION_FP32;
+    const bool lanes32 = fp32 && so.kernel_variant < 0 && so.threads_per_block == 0;
+    const size_t quad_history = lanes && !fp32 ? 0 : history_bytes(L, sizeof(double), c.sms);
+    void* history = c.history.get<unsigned char>(std::max({quad_history, lanes ? lane_history_bytes(L, c.sms, false) : 0,
+                                                           lanes32 ? lane_history_bytes(L, c.sms, true) : 0}));
     if (so.precision == UNBLENDING_PRECISION_FP64) {
         if (lanes) attach_lane_history(a, history, L, c.sms);
         else attach_history(a, history, true, v64, c.sms);
@@ -734,8 +737,12 @@ PassResult enqueue_pass(Context& c, const Spec& sp, bool refine, const unblendin
             ck(cudaMemcpyAsync(counts + 1, counts + 0, sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
         }
     } else {
-        const int variant = so.kernel_variant >= 0 ? so.kernel_variant : default_fp32_variant(L, refine);
-        attach_history(a, history, false, variant, c.sms);
+        // One pixel per lane, unless the caller names a quad variant or a block
+        // size (1024x1024, five layers, the FP32 solves of both passes: 52 + 37 ->
+        // 20 + 14 ms; bit-identical).
+        const int variant = lanes32 ? kFp32Lanes : so.kernel_variant >= 0 ? so.kernel_variant : default_fp32_variant(L, refine);
+        if (lanes32) attach_lane_history(a, history, L, c.sms, true);
+        else attach_history(a, history, false, variant, c.sms);
         a.tally = R.tally + 2;
         const Range range(refine ? "refinement solve (fp32 + fp64 re-solve)" : "first-pass solve (fp32 + fp64 re-solve)");
         ck(launch_solve_fp32(L, refine, variant, make_models<float>(layers, L), ctl32, a, threads, c.sms, s));
@@ -1197,7 +1204,7 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
                 G.v64 = lanes ? kFp64Lanes : fp64_variant(so, false);
                 const size_t quad_history =
                     lanes && so.precision == UNBLENDING_PRECISION_FP64 ? 0 : history_bytes(L, sizeof(double), c.sms);
-                void* history = plan->alloc<unsigned char>(std::max(quad_history, lanes ? lane_history_bytes(L, c.sms) : 0));
+                void* history = plan->alloc<unsigned char>(std::max(quad_history, lanes ? lane_history_bytes(L, c.sms, false) : 0));
                 auto attach_fp64 = [&](SolveArgs& x) {
                     if (lanes) attach_lane_history(x, history, L, c.sms);
                     else attach_history(x, history, true, G.v64, c.sms);
@@ -1604,8 +1611,8 @@ int32_t unblending_unmix_device_noalloc(int32_t width, int32_t height, const dou
         // whose lists leave too little room.
         const bool fp64 = so.precision == UNBLENDING_PRECISION_FP64;
         const size_t lists = fp64 ? 0 : (2 * n * sizeof(int32_t) + 255) / 256 * 256;
-        const int lane_block_count = int(std::min<size_t>(size_t(lane_blocks(L, sms)),
-                                                          (bytes - 256 - lists) / lane_block_bytes(L)));
+        const int lane_block_count = int(std::min<size_t>(size_t(lane_blocks(L, sms, false)),
+                                                          (bytes - 256 - lists) / lane_block_bytes(L, false)));
         const bool lanes = lane_solve(so) && lane_block_count >= sms / 4;
         const int v64 = lanes ? kFp64Lanes : variant_global_history(true, fp64_variant(so, false)) ? 0 : fp64_variant(so, false);
         auto attach_fp64 = [&](SolveArgs& x) {
