@@ -59,6 +59,7 @@ __host__ __device__ __forceinline__ int row_pad_shift(int w) {
 }
 __host__ __device__ __forceinline__ int padx(int x, int sh) { return x + (x >> sh); }
 constexpr int kColSegment = 128;   // rows per thread of the column pass
+constexpr int kColThreads = 64;    // small CTAs: an image of 256x256 has 17,000 threads in all
 
 // Channel value p_c of pixel i: first-pass alpha of layer c (c < L), else the
 // background colour channel c - L.
@@ -97,8 +98,9 @@ __device__ __forceinline__ double packed_value(const double* image, const double
     return m == 0 ? p : image[3 * i + (m - 1)] * p;
 }
 
-// Clamp-to-edge window mean along rows by prefix sums, one CTA per row:
-// for each plane the row's values go to shared memory, are prefix-summed
+// Clamp-to-edge window mean along rows by prefix sums, one CTA per row (few
+// rows: several, each with a share of the planes, so that an image of 256
+// rows fills the GPU too): for each plane the row's values go to shared memory, are prefix-summed
 // across the CTA (each thread scans its chunk, the chunk totals are scanned
 // by shuffles), and out[x] = (S[min(x+r, w-1)] - S[x-r-1] + clamped copies of
 // the end values) / (2r+1). PACKED: plane k of the input is packed plane k,
@@ -116,7 +118,7 @@ box_rows_prefix(const double* in, const double* image, const double* first, doub
     const int chunk = row_chunk(w);
     const int x0 = min(w, t * chunk), x1 = min(w, x0 + chunk);
     const double norm = double(2 * r + 1);
-    for (int k = 0; k < planes; ++k) {
+    for (int k = blockIdx.y; k < planes; k += gridDim.y) {
         const double* src = PACKED ? nullptr : in + size_t(k) * n + row0;
         // Coalesced load of the row into shared memory.
         for (int x = t; x < w; x += kRowThreads)
@@ -155,8 +157,13 @@ box_rows_prefix(const double* in, const double* image, const double* first, doub
 
 // Clamp-to-edge window mean along columns: one thread per (plane, column,
 // segment of kColSegment rows), sliding down its segment; the first window
-// is summed in full. Threads of a warp take adjacent columns.
-__global__ void box_cols_segments(const double* in, double* out, int w, int h, int planes, int r) {
+// is summed in full. Threads of a warp take adjacent columns. The rows that
+// enter and leave the window are read kColAhead at a time, so that their loads
+// are in flight together (the sums keep their order): a thread's serial chain
+// of loads was what the pass waited for.
+constexpr int kColAhead = 8;
+__global__ void __launch_bounds__(kColThreads) box_cols_segments(const double* __restrict__ in, double* __restrict__ out,
+                                                                 int w, int h, int planes, int r) {
     const int segs = (h + kColSegment - 1) / kColSegment;
     const size_t job = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (job >= size_t(planes) * segs * w) return;
@@ -168,10 +175,26 @@ __global__ void box_cols_segments(const double* in, double* out, int w, int h, i
     const int y0 = s * kColSegment, y1 = min(h, y0 + kColSegment);
     const double norm = double(2 * r + 1);
     double sum = 0.0;
-    for (int j = y0 - r; j <= y0 + r; ++j) sum += col[size_t(clampi(j, 0, h - 1)) * w];
-    for (int y = y0; y < y1; ++y) {
-        o[size_t(y) * w] = sum / norm;
-        sum += col[size_t(clampi(y + r + 1, 0, h - 1)) * w] - col[size_t(clampi(y - r, 0, h - 1)) * w];
+    for (int j = y0 - r; j <= y0 + r; j += kColAhead) {
+        double v[kColAhead];
+#pragma unroll
+        for (int k = 0; k < kColAhead; ++k) v[k] = col[size_t(clampi(min(j + k, y0 + r), 0, h - 1)) * w];
+#pragma unroll
+        for (int k = 0; k < kColAhead; ++k) if (j + k <= y0 + r) sum += v[k];
+    }
+    for (int y = y0; y < y1; y += kColAhead) {
+        double enter[kColAhead], leave[kColAhead];
+#pragma unroll
+        for (int k = 0; k < kColAhead; ++k) {
+            enter[k] = col[size_t(clampi(y + k + r + 1, 0, h - 1)) * w];
+            leave[k] = col[size_t(clampi(y + k - r, 0, h - 1)) * w];
+        }
+#pragma unroll
+        for (int k = 0; k < kColAhead; ++k) {
+            if (y + k >= y1) break;
+            o[size_t(y + k) * w] = sum / norm;
+            sum += enter[k] - leave[k];
+        }
     }
 }
 
@@ -262,8 +285,10 @@ cudaError_t box(const double* in, const double* image, const double* first, int 
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
             if (e != cudaSuccess) return e;
         }
-        if (image) box_rows_prefix<true><<<h, kRowThreads, smem, s>>>(nullptr, image, first, tmp, w, h, planes, L, r);
-        else box_rows_prefix<false><<<h, kRowThreads, smem, s>>>(in, nullptr, nullptr, tmp, w, h, planes, L, r);
+        const int shares = 8 * 148 / h;   // CTAs of one wave (eight per SM) per row
+        const dim3 grid(unsigned(h), unsigned(shares < 1 ? 1 : (shares > planes ? planes : shares)));
+        if (image) box_rows_prefix<true><<<grid, kRowThreads, smem, s>>>(nullptr, image, first, tmp, w, h, planes, L, r);
+        else box_rows_prefix<false><<<grid, kRowThreads, smem, s>>>(in, nullptr, nullptr, tmp, w, h, planes, L, r);
     } else {
         const int threads = 128;
         if (image) {
@@ -275,8 +300,7 @@ cudaError_t box(const double* in, const double* image, const double* first, int 
     }
     const int segs = (h + kColSegment - 1) / kColSegment;
     const size_t jobs = size_t(planes) * segs * w;
-    const int threads = 256;
-    box_cols_segments<<<unsigned((jobs + threads - 1) / threads), threads, 0, s>>>(tmp, out, w, h, planes, r);
+    box_cols_segments<<<unsigned((jobs + kColThreads - 1) / kColThreads), kColThreads, 0, s>>>(tmp, out, w, h, planes, r);
     return cudaGetLastError();
 }
 
