@@ -1135,9 +1135,10 @@ template <class T, int L, bool REFINE, bool BATCH> struct LaneSolver {
     __device__ void run() {
         const unsigned full = 0xffffffffu;
         const int total = a.list ? min(*a.list_count, a.list_limit) : (a.pixel_count >= 0 ? a.pixel_count : a.n);
-        // A small launch spreads its pixels over all warps.
-        const int warps = int(gridDim.x) * (kLaneBlock / 32);
-        if (total <= 0 || lane > (total - 1) / warps) state = kLaneIdle;
+        // A small launch spreads its pixels over all blocks, and in a block over
+        // its warps: the fewer pixels share a block's phases, the shorter the
+        // last one's chain.
+        if (total <= 0 || lane * (kLaneBlock / 32) + int(threadIdx.x >> 5) > (total - 1) / int(gridDim.x)) state = kLaneIdle;
         // Lanes waiting for each phase, one byte a phase (trial, direction,
         // gradient, outer step), counted over the block with one barrier, in
         // two buffers in turn.
