@@ -1138,7 +1138,8 @@ template <class T, int L, bool REFINE, bool BATCH> struct LaneSolver {
         // A small launch spreads its pixels over all blocks, and in a block over
         // its warps: the fewer pixels share a block's phases, the shorter the
         // last one's chain.
-        if (total <= 0 || lane * (kLaneBlock / 32) + int(threadIdx.x >> 5) > (total - 1) / int(gridDim.x)) state = kLaneIdle;
+        static_assert(kLaneBlock == 128, "four warps a block");
+        if (int64_t((threadIdx.x & 31u) << 2 | threadIdx.x >> 5) * gridDim.x >= total) state = kLaneIdle;
         // Lanes waiting for each phase, one byte a phase (trial, direction,
         // gradient, outer step), counted over the block with one barrier, in
         // two buffers in turn.
