@@ -234,9 +234,9 @@ struct Context {
     Buffer image, first, out, targets, fstatus, scratch, list_a, list_b, small, status, counters, history;
     Buffer order, order_cells;               // work-queue order of a pass (order.cu) and its counting-sort cells
     Buffer defer_list, defer_state;          // pixels deferred by an FP64 solve launch and their state
-    Buffer warm, mlp_w, mlp_b, mlp_grad;     // warm-start network on the device, its gradient
+    Buffer warm, mlp_net, mlp_grad;          // warm-start network on the device, its gradient
     Staging staging;                         // page-locked chunks for pageable caller buffers
-    std::vector<float> mlp_uploaded;         // parameters currently in mlp_w / mlp_b
+    std::vector<unsigned char> mlp_uploaded; // the network currently in mlp_net
     // Concurrent branches of a batched pass (one per layer-count group) and
     // the events that fork them from and join them to the call's stream.
     cudaStream_t branch[kMaxLayers] = {};
@@ -559,33 +559,54 @@ size_t mlp_weight_count() {
 }
 size_t mlp_bias_count() { return 3 * kMlpHidden + kMlpOut; }
 
+// Every value finite: by the exponent bits, without an exit per value (12,512
+// of them in every call that takes a network).
+bool all_finite(const float* v, int n) {
+    uint32_t worst = 0;
+    for (int i = 0; i < n; ++i) {
+        uint32_t u;
+        std::memcpy(&u, v + i, sizeof(u));
+        worst = std::max(worst, u & 0x7f800000u);
+    }
+    return worst != 0x7f800000u;
+}
+
 bool mlp_valid(const unblending_mlp* m, int L) {
     if (!m || m->struct_size < sizeof(unblending_mlp) || m->layer_count != L) return false;
-    for (int k = 0; k < 4; ++k) {
-        for (int i = 0; i < kMlpSizes[k][0] * kMlpSizes[k][1]; ++i) if (!std::isfinite(mlp_weight(*m, k)[i])) return false;
-        for (int i = 0; i < kMlpSizes[k][0]; ++i) if (!std::isfinite(mlp_bias(*m, k)[i])) return false;
-    }
+    for (int k = 0; k < 4; ++k)
+        if (!all_finite(mlp_weight(*m, k), kMlpSizes[k][0] * kMlpSizes[k][1]) || !all_finite(mlp_bias(*m, k), kMlpSizes[k][0]))
+            return false;
     return true;
 }
 
-// Device copy of a network (BF16 weights, FP32 biases), uploaded when it
-// differs from the one already on this device.
+// Device copy of a network (BF16 weights, then FP32 biases), uploaded in one
+// copy when it differs from the one already on this device.
 MlpDevice upload_model(Context& c, const unblending_mlp& m, cudaStream_t s) {
-    __nv_bfloat16* w = c.mlp_w.get<__nv_bfloat16>(mlp_weight_count());
-    float* b = c.mlp_b.get<float>(mlp_bias_count());
-    std::vector<float> flat;
-    flat.reserve(mlp_weight_count() + mlp_bias_count());
-    for (int k = 0; k < 4; ++k) flat.insert(flat.end(), mlp_weight(m, k), mlp_weight(m, k) + kMlpSizes[k][0] * kMlpSizes[k][1]);
-    for (int k = 0; k < 4; ++k) flat.insert(flat.end(), mlp_bias(m, k), mlp_bias(m, k) + kMlpSizes[k][0]);
-    if (flat != c.mlp_uploaded) {
-        std::vector<__nv_bfloat16> wb(mlp_weight_count());
-        for (size_t i = 0; i < wb.size(); ++i) wb[i] = __float2bfloat16(flat[i]);
-        ck(cudaMemcpyAsync(w, wb.data(), wb.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice, s));
-        ck(cudaMemcpyAsync(b, flat.data() + mlp_weight_count(), mlp_bias_count() * sizeof(float),
-                           cudaMemcpyHostToDevice, s));
-        ck(cudaStreamSynchronize(s));   // host staging vectors go out of scope
-        c.mlp_uploaded = std::move(flat);
+    const size_t weights = mlp_weight_count(), bytes = weights * sizeof(__nv_bfloat16) + mlp_bias_count() * sizeof(float);
+    unsigned char* base = c.mlp_net.get<unsigned char>(bytes);
+    std::vector<unsigned char> net(bytes);
+    auto* wb = reinterpret_cast<uint16_t*>(net.data());
+    auto* bias = reinterpret_cast<float*>(net.data() + weights * sizeof(uint16_t));
+    for (int k = 0; k < 4; ++k) {
+        const float* v = mlp_weight(m, k);
+        const int count = kMlpSizes[k][0] * kMlpSizes[k][1];
+        for (int i = 0; i < count; ++i) {
+            // To BF16, to nearest even (the values are finite).
+            uint32_t u;
+            std::memcpy(&u, v + i, sizeof(u));
+            wb[i] = uint16_t((u + 0x7fffu + ((u >> 16) & 1u)) >> 16);
+        }
+        wb += count;
+        std::memcpy(bias, mlp_bias(m, k), size_t(kMlpSizes[k][0]) * sizeof(float));
+        bias += kMlpSizes[k][0];
     }
+    if (net != c.mlp_uploaded) {
+        c.mlp_uploaded.clear();
+        ck(cudaMemcpyAsync(base, net.data(), bytes, cudaMemcpyHostToDevice, s));   // (pageable: staged on return)
+        c.mlp_uploaded = std::move(net);
+    }
+    const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(base);
+    const float* b = reinterpret_cast<const float*>(base + weights * sizeof(__nv_bfloat16));
     MlpDevice d;
     size_t off = 0, boff = 0;
     for (int k = 0; k < 4; ++k) {
