@@ -116,3 +116,36 @@ def test_unequal_composite_factors(cuda):
                           solver=cuda.solver_options(fp64_variant=v), stats=True)
         outs.append(out.cpu().numpy())
     np.testing.assert_array_equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("sizes", [((40, 30), (24, 50)), ((3, 2), (200, 120))])
+def test_batches_of_changing_job_lists(cuda, sizes):
+    """The batched solves' records outlive a job list: lists that take turns, on
+    two streams without a wait between the calls, and whose groups need other
+    sizes at the same place, still give the single-image results."""
+    import torch
+
+    lists, refs = [], []
+    for k, layers in enumerate(((3, 5), (6,), (5, 3))):
+        jobs, keep = [], []
+        for L in layers:
+            for w, h in sizes:
+                wl = syn.generate(w, h, [0, 1, 2, 5, 0, 3][:L], (20.0, 200.0), 10 * k + L)
+                img = torch.from_numpy(wl.image.reshape(-1)).cuda()
+                out, ref = (torch.full((4 * L * w * h,), float("nan"), dtype=torch.float64, device="cuda") for _ in range(2))
+                cuda.unmix_device(w, h, img.data_ptr(), wl.layers, ref.data_ptr())
+                jobs.append(dict(width=w, height=h, d_image=img.data_ptr(), layers=wl.layers, d_output=out.data_ptr()))
+                keep.append((img, out, ref))
+        lists.append(jobs)
+        refs.append(keep)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for turn in range(2):
+        for k, jobs in enumerate(lists):
+            cuda.unmix_batch_device(jobs, stream=streams[(turn + k) % 2].cuda_stream)
+        torch.cuda.synchronize()
+        for keep in refs:
+            for _, out, ref in keep:
+                assert torch.equal(out, ref)
+                out.fill_(float("nan"))
+        torch.cuda.synchronize()

@@ -80,7 +80,14 @@ struct Buffer {
 struct BatchPlan {
     std::vector<unsigned char> key;
     cudaGraphExec_t exec = nullptr;
-    std::vector<std::unique_ptr<Buffer>> buffers;
+    // The plan's device memory, cut from a few chunks that it takes over from
+    // the plan before: some thirty allocations and frees per new job list,
+    // several hundred MB with the lanes' records, cost more than the solves at
+    // times (two lists of ten images in turn: 53-250 ms a call, up to 1,013;
+    // kept chunks: 46-48 ms).
+    static constexpr size_t kChunk = size_t(32) << 20;
+    std::vector<std::unique_ptr<Buffer>> chunks;
+    std::vector<size_t> used;
     std::vector<int32_t*> counts;   // per group: [0] misses, [1] failures
     int64_t pixels = 0;
     int launches = 0;
@@ -89,8 +96,37 @@ struct BatchPlan {
     BatchPlan& operator=(const BatchPlan&) = delete;
     ~BatchPlan() { if (exec) cudaGraphExecDestroy(exec); }
     template <class T> T* alloc(size_t count) {
-        buffers.push_back(std::make_unique<Buffer>());
-        return buffers.back()->get<T>(count);
+        const size_t want = (std::max<size_t>(count * sizeof(T), 1) + 255) / 256 * 256;
+        size_t k = 0;
+        while (k < chunks.size() && chunks[k]->bytes - used[k] < want) ++k;
+        if (k == chunks.size()) {
+            auto fresh = std::make_unique<Buffer>();
+            fresh->get<unsigned char>(std::max(want, kChunk));
+            chunks.push_back(std::move(fresh));
+            used.push_back(0);
+        }
+        T* p = reinterpret_cast<T*>(static_cast<unsigned char*>(chunks[k]->ptr) + used[k]);
+        used[k] += want;
+        return p;
+    }
+    // The old plan's work must have ended.
+    void take_memory(BatchPlan& old) {
+        chunks = std::move(old.chunks);
+        used.assign(chunks.size(), 0);
+    }
+    // Frees the chunks that this plan left empty, once they are more than half of what it holds.
+    void give_back() {
+        size_t held = 0, empty = 0;
+        for (size_t k = 0; k < chunks.size(); ++k) {
+            held += chunks[k]->bytes;
+            if (!used[k]) empty += chunks[k]->bytes;
+        }
+        if (2 * empty <= held) return;
+        for (size_t k = chunks.size(); k-- > 0;)
+            if (!used[k]) {
+                chunks.erase(chunks.begin() + k);
+                used.erase(used.begin() + k);
+            }
     }
 };
 
@@ -242,6 +278,7 @@ struct Context {
     cudaStream_t branch[kMaxLayers] = {};
     cudaEvent_t join[kMaxLayers] = {};
     cudaEvent_t fork = nullptr;
+    cudaEvent_t batch_done = nullptr;   // the last batched pass's work: a new plan reuses its memory
     explicit Context(int dev) : device(dev) {
         ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         ck(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
@@ -1107,8 +1144,12 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
         std::lock_guard<std::mutex> lock(c.mutex);
         cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : c.stream;
         if (!c.plan || c.plan->key != key) {
-            c.plan.reset();
             auto plan = std::make_unique<BatchPlan>();
+            if (c.plan) {
+                ck(cudaEventSynchronize(c.batch_done));
+                plan->take_memory(*c.plan);
+                c.plan.reset();
+            }
             plan->key = key;
             const SolverControls ctl = controls(so), ctl32 = fp32_controls(so), ctl_re = resolve_controls(so);
             struct Group {
@@ -1225,7 +1266,8 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
                 G.v64 = lanes ? kFp64Lanes : fp64_variant(so, false);
                 const size_t quad_history =
                     lanes && so.precision == UNBLENDING_PRECISION_FP64 ? 0 : history_bytes(L, sizeof(double), c.sms);
-                void* history = plan->alloc<unsigned char>(std::max(quad_history, lanes ? lane_history_bytes(L, c.sms, false) : 0));
+                void* history = plan->alloc<unsigned char>(
+                    std::max(quad_history, lanes ? lane_history_bytes(L, c.sms, false) : 0));
                 auto attach_fp64 = [&](SolveArgs& x) {
                     if (lanes) attach_lane_history(x, history, L, c.sms);
                     else attach_history(x, history, true, G.v64, c.sms);
@@ -1283,6 +1325,7 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
             // on a 64-image batch, its one shared-memory size set by the
             // largest layer count holding every group's occupancy down.)
             if (!c.fork) {
+                ck(cudaEventCreateWithFlags(&c.batch_done, cudaEventDisableTiming));
                 ck(cudaEventCreateWithFlags(&c.fork, cudaEventDisableTiming));
                 for (int q = 0; q < kMaxLayers; ++q) {
                     ck(cudaStreamCreateWithFlags(&c.branch[q], cudaStreamNonBlocking));
@@ -1344,12 +1387,14 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
             cudaGraphDestroy(graph);
             ck(e);
             plan->launches = launches;
+            plan->give_back();
             c.plan = std::move(plan);
         }
         BatchPlan& P = *c.plan;
         ck(cudaEventRecord(c.ev[0], s));
         ck(cudaGraphLaunch(P.exec, s));
         ck(cudaEventRecord(c.ev[1], s));
+        ck(cudaEventRecord(c.batch_done, s));
         t_launches = P.launches;
         if (stats) {
             int64_t misses = 0, failed = 0;
