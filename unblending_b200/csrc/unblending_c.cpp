@@ -278,7 +278,6 @@ struct Context {
     cudaStream_t branch[kMaxLayers] = {};
     cudaEvent_t join[kMaxLayers] = {};
     cudaEvent_t fork = nullptr;
-    cudaEvent_t batch_done = nullptr;   // the last batched pass's work: a new plan reuses its memory
     explicit Context(int dev) : device(dev) {
         ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         ck(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
@@ -1146,7 +1145,9 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
         if (!c.plan || c.plan->key != key) {
             auto plan = std::make_unique<BatchPlan>();
             if (c.plan) {
-                ck(cudaEventSynchronize(c.batch_done));
+                // The whole device, as the freeing of a plan's buffers would: the
+                // last plan may also run from a graph that a caller captured.
+                ck(cudaDeviceSynchronize());
                 plan->take_memory(*c.plan);
                 c.plan.reset();
             }
@@ -1325,7 +1326,6 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
             // on a 64-image batch, its one shared-memory size set by the
             // largest layer count holding every group's occupancy down.)
             if (!c.fork) {
-                ck(cudaEventCreateWithFlags(&c.batch_done, cudaEventDisableTiming));
                 ck(cudaEventCreateWithFlags(&c.fork, cudaEventDisableTiming));
                 for (int q = 0; q < kMaxLayers; ++q) {
                     ck(cudaStreamCreateWithFlags(&c.branch[q], cudaStreamNonBlocking));
@@ -1394,7 +1394,6 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
         ck(cudaEventRecord(c.ev[0], s));
         ck(cudaGraphLaunch(P.exec, s));
         ck(cudaEventRecord(c.ev[1], s));
-        ck(cudaEventRecord(c.batch_done, s));
         t_launches = P.launches;
         if (stats) {
             int64_t misses = 0, failed = 0;
