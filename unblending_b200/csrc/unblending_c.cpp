@@ -616,8 +616,10 @@ bool mlp_valid(const unblending_mlp* m, int L) {
 }
 
 // Device copy of a network (BF16 weights, then FP32 biases), uploaded in one
-// copy when it differs from the one already on this device.
-MlpDevice upload_model(Context& c, const unblending_mlp& m, cudaStream_t s) {
+// copy when it differs from the one already on this device. A later call, on
+// any stream, takes the copy as done, so it is waited for here unless the
+// caller waits for its own work (`waits`) before it returns.
+MlpDevice upload_model(Context& c, const unblending_mlp& m, cudaStream_t s, bool waits = false) {
     const size_t weights = mlp_weight_count(), bytes = weights * sizeof(__nv_bfloat16) + mlp_bias_count() * sizeof(float);
     unsigned char* base = c.mlp_net.get<unsigned char>(bytes);
     std::vector<unsigned char> net(bytes);
@@ -638,7 +640,8 @@ MlpDevice upload_model(Context& c, const unblending_mlp& m, cudaStream_t s) {
     }
     if (net != c.mlp_uploaded) {
         c.mlp_uploaded.clear();
-        ck(cudaMemcpyAsync(base, net.data(), bytes, cudaMemcpyHostToDevice, s));   // (pageable: staged on return)
+        ck(cudaMemcpyAsync(base, net.data(), bytes, cudaMemcpyHostToDevice, s));
+        if (!waits) ck(cudaStreamSynchronize(s));
         c.mlp_uploaded = std::move(net);
     }
     const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(base);
@@ -1426,7 +1429,7 @@ int32_t unblending_mlp_predict_device(const unblending_mlp* model, int32_t width
         Context& c = context();
         std::lock_guard<std::mutex> lock(c.mutex);
         cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : c.stream;
-        const MlpDevice dev = upload_model(c, *model, s);
+        const MlpDevice dev = upload_model(c, *model, s, true);
         int32_t* err = c.small.get<int32_t>(8) + 7;
         ck(cudaMemsetAsync(err, 0, sizeof(int32_t), s));
         ck(launch_mlp_infer(dev, image, width, height, model->layer_count, out, err, c.sms, s));
@@ -1451,7 +1454,7 @@ int32_t unblending_mlp_loss_grad_device(const unblending_mlp* model, int32_t cou
         Context& c = context();
         std::lock_guard<std::mutex> lock(c.mutex);
         cudaStream_t s = c.stream;
-        const MlpDevice dev = upload_model(c, *model, s);
+        const MlpDevice dev = upload_model(c, *model, s, true);
         const size_t nw = mlp_weight_count(), nb = mlp_bias_count(), np = nw + nb;
         float* grad = c.mlp_grad.get<float>(np + 1);
         ck(cudaMemsetAsync(grad, 0, (np + 1) * sizeof(float), s));
