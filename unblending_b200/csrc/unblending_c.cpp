@@ -1131,6 +1131,8 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
     put(&so.frozen_stop, sizeof(so.frozen_stop));
     put(&so.pixel_order, sizeof(so.pixel_order));
     put(&so.defer_outer, sizeof(so.defer_outer));
+    const unsigned char opaque = specs[0].opaque;   // (one options struct for all jobs)
+    put(&opaque, sizeof(opaque));
     for (int k = 0; k < count; ++k) {
         const auto& J = jobs[k];
         put(&J.width, sizeof(J.width)); put(&J.height, sizeof(J.height));
