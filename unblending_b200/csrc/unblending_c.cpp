@@ -617,9 +617,12 @@ bool mlp_valid(const unblending_mlp* m, int L) {
 
 // Device copy of a network (BF16 weights, then FP32 biases), uploaded in one
 // copy when it differs from the one already on this device. A later call, on
-// any stream, takes the copy as done, so it is waited for here unless the
-// caller waits for its own work (`waits`) before it returns.
-MlpDevice upload_model(Context& c, const unblending_mlp& m, cudaStream_t s, bool waits = false) {
+// any stream, takes the recorded network as uploaded, so it is recorded only
+// once its copy was waited for: here, or by the caller, whose own wait at its
+// end covers the copy and who then calls `model_uploaded` (a call that fails
+// before, in a stream capture for instance, leaves no network recorded).
+MlpDevice upload_model(Context& c, const unblending_mlp& m, cudaStream_t s,
+                       std::vector<unsigned char>* pending = nullptr) {
     const size_t weights = mlp_weight_count(), bytes = weights * sizeof(__nv_bfloat16) + mlp_bias_count() * sizeof(float);
     unsigned char* base = c.mlp_net.get<unsigned char>(bytes);
     std::vector<unsigned char> net(bytes);
@@ -641,8 +644,12 @@ MlpDevice upload_model(Context& c, const unblending_mlp& m, cudaStream_t s, bool
     if (net != c.mlp_uploaded) {
         c.mlp_uploaded.clear();
         ck(cudaMemcpyAsync(base, net.data(), bytes, cudaMemcpyHostToDevice, s));
-        if (!waits) ck(cudaStreamSynchronize(s));
-        c.mlp_uploaded = std::move(net);
+        if (pending) {
+            *pending = std::move(net);
+        } else {
+            ck(cudaStreamSynchronize(s));
+            c.mlp_uploaded = std::move(net);
+        }
     }
     const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(base);
     const float* b = reinterpret_cast<const float*>(base + weights * sizeof(__nv_bfloat16));
@@ -653,6 +660,10 @@ MlpDevice upload_model(Context& c, const unblending_mlp& m, cudaStream_t s, bool
         d.b[k] = b + boff; boff += kMlpSizes[k][0];
     }
     return d;
+}
+
+void model_uploaded(Context& c, std::vector<unsigned char>& pending) {
+    if (!pending.empty()) c.mlp_uploaded = std::move(pending);
 }
 
 // --------------------------------------------------------------- a pass --
@@ -1431,7 +1442,8 @@ int32_t unblending_mlp_predict_device(const unblending_mlp* model, int32_t width
         Context& c = context();
         std::lock_guard<std::mutex> lock(c.mutex);
         cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : c.stream;
-        const MlpDevice dev = upload_model(c, *model, s, true);
+        std::vector<unsigned char> pending;
+        const MlpDevice dev = upload_model(c, *model, s, &pending);
         int32_t* err = c.small.get<int32_t>(8) + 7;
         ck(cudaMemsetAsync(err, 0, sizeof(int32_t), s));
         ck(launch_mlp_infer(dev, image, width, height, model->layer_count, out, err, c.sms, s));
@@ -1439,6 +1451,7 @@ int32_t unblending_mlp_predict_device(const unblending_mlp* model, int32_t width
         int32_t failed = 0;
         ck(cudaMemcpyAsync(&failed, err, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
         ck(cudaStreamSynchronize(s));
+        model_uploaded(c, pending);
         if (failed) throw CudaFailure(cudaErrorLaunchTimeout);
         return UNBLENDING_OK;
     });
@@ -1456,7 +1469,8 @@ int32_t unblending_mlp_loss_grad_device(const unblending_mlp* model, int32_t cou
         Context& c = context();
         std::lock_guard<std::mutex> lock(c.mutex);
         cudaStream_t s = c.stream;
-        const MlpDevice dev = upload_model(c, *model, s, true);
+        std::vector<unsigned char> pending;
+        const MlpDevice dev = upload_model(c, *model, s, &pending);
         const size_t nw = mlp_weight_count(), nb = mlp_bias_count(), np = nw + nb;
         float* grad = c.mlp_grad.get<float>(np + 1);
         ck(cudaMemsetAsync(grad, 0, (np + 1) * sizeof(float), s));
@@ -1476,6 +1490,7 @@ int32_t unblending_mlp_loss_grad_device(const unblending_mlp* model, int32_t cou
         ck(cudaMemcpyAsync(out.data(), grad, (np + 1) * sizeof(float), cudaMemcpyDeviceToHost, s));
         ck(cudaMemcpyAsync(&failed, err, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
         ck(cudaStreamSynchronize(s));
+        model_uploaded(c, pending);
         if (failed) throw CudaFailure(cudaErrorLaunchTimeout);
         gradient->layer_count = model->layer_count;
         o = 0;
