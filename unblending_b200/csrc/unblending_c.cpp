@@ -80,6 +80,7 @@ struct Buffer {
 struct BatchPlan {
     std::vector<unsigned char> key;
     cudaGraphExec_t exec = nullptr;
+    cudaEvent_t done = nullptr;     // after the last replay (all on the key's stream)
     // The plan's device memory, cut from a few chunks that it takes over from
     // the plan before: some thirty allocations and frees per new job list,
     // several hundred MB with the lanes' records, cost more than the solves at
@@ -94,7 +95,10 @@ struct BatchPlan {
     BatchPlan() = default;
     BatchPlan(const BatchPlan&) = delete;
     BatchPlan& operator=(const BatchPlan&) = delete;
-    ~BatchPlan() { if (exec) cudaGraphExecDestroy(exec); }
+    ~BatchPlan() {
+        if (exec) cudaGraphExecDestroy(exec);
+        if (done) cudaEventDestroy(done);
+    }
     template <class T> T* alloc(size_t count) {
         const size_t want = (std::max<size_t>(count * sizeof(T), 1) + 255) / 256 * 256;
         size_t k = 0;
@@ -1161,9 +1165,11 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
         if (!c.plan || c.plan->key != key) {
             auto plan = std::make_unique<BatchPlan>();
             if (c.plan) {
-                // The whole device, as the freeing of a plan's buffers would: the
-                // last plan may also run from a graph that a caller captured.
-                ck(cudaDeviceSynchronize());
+                // The last plan's memory, once its last replay has ended (its graph
+                // is launched here alone: a stream capture refuses it). A wait for
+                // the device would be refused, and end the capture, while any other
+                // stream captures.
+                ck(cudaEventSynchronize(c.plan->done));
                 plan->take_memory(*c.plan);
                 c.plan.reset();
             }
@@ -1402,6 +1408,7 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
             cudaError_t e = cudaGraphInstantiate(&plan->exec, graph, 0);
             cudaGraphDestroy(graph);
             ck(e);
+            ck(cudaEventCreateWithFlags(&plan->done, cudaEventDisableTiming));
             plan->launches = launches;
             plan->give_back();
             c.plan = std::move(plan);
@@ -1409,6 +1416,7 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
         BatchPlan& P = *c.plan;
         ck(cudaEventRecord(c.ev[0], s));
         ck(cudaGraphLaunch(P.exec, s));
+        ck(cudaEventRecord(P.done, s));
         ck(cudaEventRecord(c.ev[1], s));
         t_launches = P.launches;
         if (stats) {
