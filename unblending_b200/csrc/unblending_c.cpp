@@ -23,6 +23,7 @@
 
 #include "../../include/unblending.h"
 #include "../../include/unblending_b200.h"
+#include "plan_memory.hpp"
 #include "solver_dispatch.hpp"
 
 namespace {
@@ -81,14 +82,7 @@ struct BatchPlan {
     std::vector<unsigned char> key;
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t done = nullptr;     // after the last replay (all on the key's stream)
-    // The plan's device memory, cut from a few chunks that it takes over from
-    // the plan before: some thirty allocations and frees per new job list,
-    // several hundred MB with the lanes' records, cost more than the solves at
-    // times (two lists of ten images in turn: 53-250 ms a call, up to 1,013;
-    // kept chunks: 46-48 ms).
-    static constexpr size_t kChunk = size_t(32) << 20;
-    std::vector<std::unique_ptr<Buffer>> chunks;
-    std::vector<size_t> used;
+    PlanMemory<Buffer> memory;
     std::vector<int32_t*> counts;   // per group: [0] misses, [1] failures
     int64_t pixels = 0;
     int launches = 0;
@@ -98,39 +92,6 @@ struct BatchPlan {
     ~BatchPlan() {
         if (exec) cudaGraphExecDestroy(exec);
         if (done) cudaEventDestroy(done);
-    }
-    template <class T> T* alloc(size_t count) {
-        const size_t want = (std::max<size_t>(count * sizeof(T), 1) + 255) / 256 * 256;
-        size_t k = 0;
-        while (k < chunks.size() && chunks[k]->bytes - used[k] < want) ++k;
-        if (k == chunks.size()) {
-            auto fresh = std::make_unique<Buffer>();
-            fresh->get<unsigned char>(std::max(want, kChunk));
-            chunks.push_back(std::move(fresh));
-            used.push_back(0);
-        }
-        T* p = reinterpret_cast<T*>(static_cast<unsigned char*>(chunks[k]->ptr) + used[k]);
-        used[k] += want;
-        return p;
-    }
-    // The old plan's work must have ended.
-    void take_memory(BatchPlan& old) {
-        chunks = std::move(old.chunks);
-        used.assign(chunks.size(), 0);
-    }
-    // Frees the chunks that this plan left empty, once they are more than half of what it holds.
-    void give_back() {
-        size_t held = 0, empty = 0;
-        for (size_t k = 0; k < chunks.size(); ++k) {
-            held += chunks[k]->bytes;
-            if (!used[k]) empty += chunks[k]->bytes;
-        }
-        if (2 * empty <= held) return;
-        for (size_t k = chunks.size(); k-- > 0;)
-            if (!used[k]) {
-                chunks.erase(chunks.begin() + k);
-                used.erase(used.begin() + k);
-            }
     }
 };
 
@@ -1163,255 +1124,254 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
         std::lock_guard<std::mutex> lock(c.mutex);
         cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : c.stream;
         if (!c.plan || c.plan->key != key) {
-            auto plan = std::make_unique<BatchPlan>();
-            if (c.plan) {
-                // The last plan's memory, once its last replay has ended (its graph
-                // is launched here alone: a stream capture refuses it). A wait for
-                // the device would be refused, and end the capture, while any other
-                // stream captures.
-                ck(cudaEventSynchronize(c.plan->done));
-                plan->take_memory(*c.plan);
-                c.plan.reset();
-            }
-            plan->key = key;
-            const SolverControls ctl = controls(so), ctl32 = fp32_controls(so), ctl_re = resolve_controls(so);
-            struct Group {
-                int L;
-                SolveArgs fp, mid, re;   // first solve (warm where given), FP32 re-solve of its misses from
-                                         // the reference start (groups with a learned start), FP64 re-solve
-                uint32_t* queues;
-                int32_t* counts;
-                std::vector<std::pair<int, float*>> infer;   // job, warm slice
-                MlpDevice net;
-                int variant = 0, threads = 128;
-                int v64 = 0;                // FP64 kernel of the group's solve or re-solve
-                int64_t total = 0;
-                int32_t* order = nullptr;   // colour order of the group's queue (pixel_order)
-                uint32_t* order_cells = nullptr;
-            };
-            std::vector<Group> gs;
-            for (auto& [L, members] : groups) {
-                Group G;
-                G.L = L;
-                std::vector<BatchJob> table, cold;
-                std::vector<Models<float>> m32;
-                std::vector<Models<double>> m64;
-                int64_t off = 0;
-                const unblending_mlp* net = group_model.count(L) ? group_model[L] : nullptr;
-                float* warm = nullptr;
-                int64_t total = 0;
-                for (int k : members) total += int64_t(specs[k].pixels);
-                G.total = total;
-                if (net) warm = plan->alloc<float>(size_t(total) * 4 * L);
-                for (int k : members) {
-                    const auto& J = jobs[k];
-                    BatchJob b;
-                    b.image = J.image; b.out = J.output; b.status = J.status;
-                    b.offset = off; b.n = int64_t(specs[k].pixels); b.model = int32_t(table.size());
-                    b.warm = nullptr;
-                    cold.push_back(b);
-                    if (J.warm_start) {
-                        b.warm = warm + off * 4 * L;
-                        G.infer.emplace_back(k, const_cast<float*>(b.warm));
-                    }
-                    table.push_back(b);
-                    m32.push_back(make_models<float>(J.layers, L));
-                    m64.push_back(make_models<double>(J.layers, L));
-                    off += b.n;
-                }
-                if (net) {
-                    // The group's own device copy of its network (the graph keeps referring to it).
-                    const MlpDevice shared = upload_model(c, *net, s);
-                    __nv_bfloat16* w = plan->alloc<__nv_bfloat16>(mlp_weight_count());
-                    float* bb = plan->alloc<float>(mlp_bias_count());
-                    ck(cudaMemcpyAsync(w, shared.w[0], mlp_weight_count() * sizeof(__nv_bfloat16),
-                                       cudaMemcpyDeviceToDevice, s));
-                    ck(cudaMemcpyAsync(bb, shared.b[0], mlp_bias_count() * sizeof(float), cudaMemcpyDeviceToDevice, s));
-                    for (int q = 0; q < 4; ++q) {
-                        G.net.w[q] = w + (shared.w[q] - shared.w[0]);
-                        G.net.b[q] = bb + (shared.b[q] - shared.b[0]);
-                    }
-                }
-                BatchJob* d_table = plan->alloc<BatchJob>(2 * table.size());
-                Models<float>* d_m32 = plan->alloc<Models<float>>(m32.size());
-                Models<double>* d_m64 = plan->alloc<Models<double>>(m64.size());
-                ck(cudaMemcpyAsync(d_table, table.data(), table.size() * sizeof(BatchJob), cudaMemcpyHostToDevice, s));
-                ck(cudaMemcpyAsync(d_table + table.size(), cold.data(), cold.size() * sizeof(BatchJob),
-                                   cudaMemcpyHostToDevice, s));
-                ck(cudaMemcpyAsync(d_m32, m32.data(), m32.size() * sizeof(Models<float>), cudaMemcpyHostToDevice, s));
-                ck(cudaMemcpyAsync(d_m64, m64.data(), m64.size() * sizeof(Models<double>), cudaMemcpyHostToDevice, s));
-                ck(cudaStreamSynchronize(s));   // host tables go out of scope
-                G.queues = plan->alloc<uint32_t>(8);
-                G.counts = reinterpret_cast<int32_t*>(G.queues + 4);
-                int32_t* lists = plan->alloc<int32_t>(2 * size_t(total));
-                if (so.pixel_order) {
-                    G.order = plan->alloc<int32_t>(size_t(total));
-                    G.order_cells = plan->alloc<uint32_t>(order_cells(int(total)));
-                }
-                SolveArgs& a = G.fp;
-                a.n = int(total);
-                a.jobs = d_table; a.job_count = int(table.size());
-                a.opaque = specs[members[0]].opaque; a.smooth = 0;
-                a.queue = G.queues;
-                a.miss_list = lists; a.miss_count = G.counts + 0;
-                a.order = G.order;
-                SolveArgs& b = G.re;
-                b = a;
-                b.order = nullptr;
-                b.jobs = d_table + table.size();
-                b.models = d_m64;
-                b.list = lists; b.list_count = G.counts + 0;
-                b.miss_list = lists + total; b.miss_count = G.counts + 1;
-                b.queue = G.queues + 1;
-                if (!G.infer.empty() && so.precision != UNBLENDING_PRECISION_FP64) {
-                    // As the single-image pass: the learned start's misses get the
-                    // plain FP32 solve first (cold jobs of the group repeat theirs,
-                    // with the same result), its misses the FP64 re-solve.
-                    SolveArgs& w = G.mid;
-                    w = a;
-                    w.order = nullptr;
-                    w.jobs = d_table + table.size();
-                    w.models = d_m32;
-                    w.list = lists; w.list_count = G.counts + 0;
-                    w.miss_list = lists + total; w.miss_count = reinterpret_cast<int32_t*>(G.queues + 3);
-                    w.queue = G.queues + 2;
-                    b.list = lists + total; b.list_count = w.miss_count;
-                    b.miss_list = lists;
-                }
-                a.models = so.precision == UNBLENDING_PRECISION_FP64 ? static_cast<const void*>(d_m64) : d_m32;
-                // FP64: the solve's misses are the group's failures, unless a
-                // learned start leaves them to the plain solve (G.re, as the
-                // single-image pass does).
-                if (so.precision == UNBLENDING_PRECISION_FP64 && G.infer.empty()) a.miss_count = G.counts + 1;
-                plan->counts.push_back(G.counts);
-                plan->pixels += total;
-                const bool lanes = lane_solve(so);
-                G.v64 = lanes ? kFp64Lanes : fp64_variant(so, false);
-                const size_t quad_history =
-                    lanes && so.precision == UNBLENDING_PRECISION_FP64 ? 0 : history_bytes(L, sizeof(double), c.sms);
-                void* history = plan->alloc<unsigned char>(
-                    std::max(quad_history, lanes ? lane_history_bytes(L, c.sms, false) : 0));
-                auto attach_fp64 = [&](SolveArgs& x) {
-                    if (lanes) attach_lane_history(x, history, L, c.sms);
-                    else attach_history(x, history, true, G.v64, c.sms);
+            // The last plan's memory is taken over once its last replay has ended
+            // (its graph is launched here alone: a stream capture refuses it). A
+            // wait for the device would be refused, and end the capture, while any
+            // other stream captures.
+            if (c.plan) ck(cudaEventSynchronize(c.plan->done));
+            c.plan = next_plan(c.plan, [&](BatchPlan& plan) {
+                plan.key = key;
+                const SolverControls ctl = controls(so), ctl32 = fp32_controls(so), ctl_re = resolve_controls(so);
+                struct Group {
+                    int L;
+                    SolveArgs fp, mid, re;   // first solve (warm where given), FP32 re-solve of its misses from
+                                             // the reference start (groups with a learned start), FP64 re-solve
+                    uint32_t* queues;
+                    int32_t* counts;
+                    std::vector<std::pair<int, float*>> infer;   // job, warm slice
+                    MlpDevice net;
+                    int variant = 0, threads = 128;
+                    int v64 = 0;                // FP64 kernel of the group's solve or re-solve
+                    int64_t total = 0;
+                    int32_t* order = nullptr;   // colour order of the group's queue (pixel_order)
+                    uint32_t* order_cells = nullptr;
                 };
-                // Autotuner: time each FP32 kernel variant / block size on a
-                // sample of this group's pixels spread over its images.
-                const auto tkey = std::make_pair(L, so.precision);
-                if (so.precision == UNBLENDING_PRECISION_FP32 && so.threads_per_block == 0 && so.kernel_variant < 0) {
-                    if (!c.tuned.count(tkey)) {
-                        const int S = int(std::min<int64_t>(total, 8192));
-                        std::vector<int32_t> sample(S);
-                        for (int q = 0; q < S; ++q) sample[q] = int32_t(int64_t(q) * total / S);
-                        int32_t* d_sample = plan->alloc<int32_t>(S);
-                        int32_t* d_count = plan->alloc<int32_t>(1);
-                        ck(cudaMemcpyAsync(d_sample, sample.data(), S * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-                        ck(cudaMemcpyAsync(d_count, &S, sizeof(int32_t), cudaMemcpyHostToDevice, s));
-                        const std::pair<int, int> candidates[4] = {{3, 128}, {1, 128}, {2, 128}, {3, 64}};
-                        float best_ms = 1e30f;
-                        std::pair<int, int> best = candidates[0];
-                        for (const auto& cand : candidates) {
-                            SolveArgs t = a;
-                            t.jobs = d_table + table.size();   // reference start: the network has not run yet
-                            t.list = d_sample; t.list_count = d_count;
-                            t.miss_list = nullptr; t.status = nullptr;
-                            attach_history(t, history, false, cand.first, c.sms);
-                            ck(cudaMemsetAsync(G.queues, 0, 8 * sizeof(uint32_t), s));
-                            ck(cudaEventRecord(c.ev[4], s));
-                            ck(launch_solve_batch_fp32(L, cand.first, ctl32, t, cand.second, c.sms, s));
-                            ck(cudaEventRecord(c.ev[5], s));
-                            ck(cudaEventSynchronize(c.ev[5]));
-                            const float ms = elapsed(c.ev[4], c.ev[5]);
-                            if (ms < best_ms) { best_ms = ms; best = cand; }
+                std::vector<Group> gs;
+                for (auto& [L, members] : groups) {
+                    Group G;
+                    G.L = L;
+                    std::vector<BatchJob> table, cold;
+                    std::vector<Models<float>> m32;
+                    std::vector<Models<double>> m64;
+                    int64_t off = 0;
+                    const unblending_mlp* net = group_model.count(L) ? group_model[L] : nullptr;
+                    float* warm = nullptr;
+                    int64_t total = 0;
+                    for (int k : members) total += int64_t(specs[k].pixels);
+                    G.total = total;
+                    if (net) warm = plan.memory.alloc<float>(size_t(total) * 4 * L);
+                    for (int k : members) {
+                        const auto& J = jobs[k];
+                        BatchJob b;
+                        b.image = J.image; b.out = J.output; b.status = J.status;
+                        b.offset = off; b.n = int64_t(specs[k].pixels); b.model = int32_t(table.size());
+                        b.warm = nullptr;
+                        cold.push_back(b);
+                        if (J.warm_start) {
+                            b.warm = warm + off * 4 * L;
+                            G.infer.emplace_back(k, const_cast<float*>(b.warm));
                         }
-                        c.tuned[tkey] = best;
+                        table.push_back(b);
+                        m32.push_back(make_models<float>(J.layers, L));
+                        m64.push_back(make_models<double>(J.layers, L));
+                        off += b.n;
                     }
-                    G.variant = c.tuned[tkey].first;
-                    G.threads = c.tuned[tkey].second;
-                } else {
-                    G.variant = so.kernel_variant >= 0 ? so.kernel_variant : default_fp32_variant(L, false);
-                    G.threads = so.threads_per_block ? so.threads_per_block : 128;
-                }
-                if (so.precision == UNBLENDING_PRECISION_FP64) attach_fp64(a);
-                else attach_history(a, history, false, G.variant, c.sms);
-                attach_history(G.mid, history, false, G.variant, c.sms);
-                attach_fp64(b);
-                gs.push_back(G);
-            }
-            // Capture every group's work into one graph, each group on its own
-            // branch: the groups' persistent launches run back to back on the
-            // GPU, the next group's blocks filling the SMs that the previous
-            // group's tail frees. (One kernel over all layer counts was built
-            // and measured twice: with every solver inlined, its single
-            // register allocation spilled 0.6-1.6 KB of stack per thread; with
-            // each count's solver out of line, it ran 4.45 against 6.52 Mpx/s
-            // on a 64-image batch, its one shared-memory size set by the
-            // largest layer count holding every group's occupancy down.)
-            if (!c.fork) {
-                ck(cudaEventCreateWithFlags(&c.fork, cudaEventDisableTiming));
-                for (int q = 0; q < kMaxLayers; ++q) {
-                    ck(cudaStreamCreateWithFlags(&c.branch[q], cudaStreamNonBlocking));
-                    ck(cudaEventCreateWithFlags(&c.join[q], cudaEventDisableTiming));
-                }
-            }
-            cudaGraph_t graph = nullptr;
-            ck(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
-            int launches = 0;
-            try {
-                ck(cudaEventRecord(c.fork, s));
-                for (size_t gi = 0; gi < gs.size(); ++gi) {
-                    auto& G = gs[gi];
-                    cudaStream_t s = c.branch[gi];   // this group's branch (shadows the call's stream)
-                    ck(cudaStreamWaitEvent(s, c.fork, 0));
-                    ck(cudaMemsetAsync(G.queues, 0, 8 * sizeof(uint32_t), s));
-                    if (G.order) {
-                        // The group's queue grouped by colour (order.cu).
-                        ck(launch_group_order(G.fp.jobs, G.fp.job_count, int(G.total), G.order_cells, G.order, c.sms,
-                                              s));
-                        launches += 4;
-                    }
-                    for (auto& [k, w] : G.infer) {
-                        ck(launch_mlp_infer(G.net, jobs[k].image, jobs[k].width, jobs[k].height, G.L, w, G.counts + 3,
-                                            c.sms, s));
-                        ++launches;
-                    }
-                    if (so.precision == UNBLENDING_PRECISION_FP64) {
-                        ck(launch_solve_batch_fp64(G.L, G.v64, ctl, G.fp, 128, c.sms, s));
-                        ++launches;
-                        if (!G.infer.empty()) {
-                            ck(launch_solve_batch_fp64(G.L, G.v64, ctl, G.re, 128, c.sms, s));
-                            ++launches;
+                    if (net) {
+                        // The group's own device copy of its network (the graph keeps referring to it).
+                        const MlpDevice shared = upload_model(c, *net, s);
+                        __nv_bfloat16* w = plan.memory.alloc<__nv_bfloat16>(mlp_weight_count());
+                        float* bb = plan.memory.alloc<float>(mlp_bias_count());
+                        ck(cudaMemcpyAsync(w, shared.w[0], mlp_weight_count() * sizeof(__nv_bfloat16),
+                                           cudaMemcpyDeviceToDevice, s));
+                        ck(cudaMemcpyAsync(bb, shared.b[0], mlp_bias_count() * sizeof(float),
+                                           cudaMemcpyDeviceToDevice, s));
+                        for (int q = 0; q < 4; ++q) {
+                            G.net.w[q] = w + (shared.w[q] - shared.w[0]);
+                            G.net.b[q] = bb + (shared.b[q] - shared.b[0]);
                         }
+                    }
+                    BatchJob* d_table = plan.memory.alloc<BatchJob>(2 * table.size());
+                    Models<float>* d_m32 = plan.memory.alloc<Models<float>>(m32.size());
+                    Models<double>* d_m64 = plan.memory.alloc<Models<double>>(m64.size());
+                    ck(cudaMemcpyAsync(d_table, table.data(), table.size() * sizeof(BatchJob),
+                                       cudaMemcpyHostToDevice, s));
+                    ck(cudaMemcpyAsync(d_table + table.size(), cold.data(), cold.size() * sizeof(BatchJob),
+                                       cudaMemcpyHostToDevice, s));
+                    ck(cudaMemcpyAsync(d_m32, m32.data(), m32.size() * sizeof(Models<float>),
+                                       cudaMemcpyHostToDevice, s));
+                    ck(cudaMemcpyAsync(d_m64, m64.data(), m64.size() * sizeof(Models<double>),
+                                       cudaMemcpyHostToDevice, s));
+                    ck(cudaStreamSynchronize(s));   // host tables go out of scope
+                    G.queues = plan.memory.alloc<uint32_t>(8);
+                    G.counts = reinterpret_cast<int32_t*>(G.queues + 4);
+                    int32_t* lists = plan.memory.alloc<int32_t>(2 * size_t(total));
+                    if (so.pixel_order) {
+                        G.order = plan.memory.alloc<int32_t>(size_t(total));
+                        G.order_cells = plan.memory.alloc<uint32_t>(order_cells(int(total)));
+                    }
+                    SolveArgs& a = G.fp;
+                    a.n = int(total);
+                    a.jobs = d_table; a.job_count = int(table.size());
+                    a.opaque = specs[members[0]].opaque; a.smooth = 0;
+                    a.queue = G.queues;
+                    a.miss_list = lists; a.miss_count = G.counts + 0;
+                    a.order = G.order;
+                    SolveArgs& b = G.re;
+                    b = a;
+                    b.order = nullptr;
+                    b.jobs = d_table + table.size();
+                    b.models = d_m64;
+                    b.list = lists; b.list_count = G.counts + 0;
+                    b.miss_list = lists + total; b.miss_count = G.counts + 1;
+                    b.queue = G.queues + 1;
+                    if (!G.infer.empty() && so.precision != UNBLENDING_PRECISION_FP64) {
+                        // As the single-image pass: the learned start's misses get the
+                        // plain FP32 solve first (cold jobs of the group repeat theirs,
+                        // with the same result), its misses the FP64 re-solve.
+                        SolveArgs& w = G.mid;
+                        w = a;
+                        w.order = nullptr;
+                        w.jobs = d_table + table.size();
+                        w.models = d_m32;
+                        w.list = lists; w.list_count = G.counts + 0;
+                        w.miss_list = lists + total; w.miss_count = reinterpret_cast<int32_t*>(G.queues + 3);
+                        w.queue = G.queues + 2;
+                        b.list = lists + total; b.list_count = w.miss_count;
+                        b.miss_list = lists;
+                    }
+                    a.models = so.precision == UNBLENDING_PRECISION_FP64 ? static_cast<const void*>(d_m64) : d_m32;
+                    // FP64: the solve's misses are the group's failures, unless a
+                    // learned start leaves them to the plain solve (G.re, as the
+                    // single-image pass does).
+                    if (so.precision == UNBLENDING_PRECISION_FP64 && G.infer.empty()) a.miss_count = G.counts + 1;
+                    plan.counts.push_back(G.counts);
+                    plan.pixels += total;
+                    const bool lanes = lane_solve(so);
+                    G.v64 = lanes ? kFp64Lanes : fp64_variant(so, false);
+                    const size_t quad_history =
+                        lanes && so.precision == UNBLENDING_PRECISION_FP64 ? 0 : history_bytes(L, sizeof(double), c.sms);
+                    void* history = plan.memory.alloc<unsigned char>(
+                        std::max(quad_history, lanes ? lane_history_bytes(L, c.sms, false) : 0));
+                    auto attach_fp64 = [&](SolveArgs& x) {
+                        if (lanes) attach_lane_history(x, history, L, c.sms);
+                        else attach_history(x, history, true, G.v64, c.sms);
+                    };
+                    // Autotuner: time each FP32 kernel variant / block size on a
+                    // sample of this group's pixels spread over its images.
+                    const auto tkey = std::make_pair(L, so.precision);
+                    if (so.precision == UNBLENDING_PRECISION_FP32 && so.threads_per_block == 0 && so.kernel_variant < 0) {
+                        if (!c.tuned.count(tkey)) {
+                            const int S = int(std::min<int64_t>(total, 8192));
+                            std::vector<int32_t> sample(S);
+                            for (int q = 0; q < S; ++q) sample[q] = int32_t(int64_t(q) * total / S);
+                            int32_t* d_sample = plan.memory.alloc<int32_t>(S);
+                            int32_t* d_count = plan.memory.alloc<int32_t>(1);
+                            ck(cudaMemcpyAsync(d_sample, sample.data(), S * sizeof(int32_t), cudaMemcpyHostToDevice, s));
+                            ck(cudaMemcpyAsync(d_count, &S, sizeof(int32_t), cudaMemcpyHostToDevice, s));
+                            const std::pair<int, int> candidates[4] = {{3, 128}, {1, 128}, {2, 128}, {3, 64}};
+                            float best_ms = 1e30f;
+                            std::pair<int, int> best = candidates[0];
+                            for (const auto& cand : candidates) {
+                                SolveArgs t = a;
+                                t.jobs = d_table + table.size();   // reference start: the network has not run yet
+                                t.list = d_sample; t.list_count = d_count;
+                                t.miss_list = nullptr; t.status = nullptr;
+                                attach_history(t, history, false, cand.first, c.sms);
+                                ck(cudaMemsetAsync(G.queues, 0, 8 * sizeof(uint32_t), s));
+                                ck(cudaEventRecord(c.ev[4], s));
+                                ck(launch_solve_batch_fp32(L, cand.first, ctl32, t, cand.second, c.sms, s));
+                                ck(cudaEventRecord(c.ev[5], s));
+                                ck(cudaEventSynchronize(c.ev[5]));
+                                const float ms = elapsed(c.ev[4], c.ev[5]);
+                                if (ms < best_ms) { best_ms = ms; best = cand; }
+                            }
+                            c.tuned[tkey] = best;
+                        }
+                        G.variant = c.tuned[tkey].first;
+                        G.threads = c.tuned[tkey].second;
                     } else {
-                        ck(launch_solve_batch_fp32(G.L, G.variant, ctl32, G.fp, G.threads, c.sms, s));
-                        ++launches;
-                        if (so.resolve_misses && !G.infer.empty()) {
-                            ck(launch_solve_batch_fp32(G.L, G.variant, ctl32, G.mid, G.threads, c.sms, s));
-                            ++launches;
-                        }
-                        if (so.resolve_misses) {
-                            ck(launch_solve_batch_fp64(G.L, G.v64, ctl_re, G.re, 128, c.sms, s));
-                            ++launches;
-                        } else {
-                            ck(cudaMemcpyAsync(G.counts + 1, G.counts, sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
-                        }
+                        G.variant = so.kernel_variant >= 0 ? so.kernel_variant : default_fp32_variant(L, false);
+                        G.threads = so.threads_per_block ? so.threads_per_block : 128;
                     }
-                    ck(cudaEventRecord(c.join[gi], s));
+                    if (so.precision == UNBLENDING_PRECISION_FP64) attach_fp64(a);
+                    else attach_history(a, history, false, G.variant, c.sms);
+                    attach_history(G.mid, history, false, G.variant, c.sms);
+                    attach_fp64(b);
+                    gs.push_back(G);
                 }
-                for (size_t gi = 0; gi < gs.size(); ++gi) ck(cudaStreamWaitEvent(s, c.join[gi], 0));
-            } catch (...) {
-                cudaStreamEndCapture(s, &graph);
-                if (graph) cudaGraphDestroy(graph);
-                throw;
-            }
-            ck(cudaStreamEndCapture(s, &graph));
-            cudaError_t e = cudaGraphInstantiate(&plan->exec, graph, 0);
-            cudaGraphDestroy(graph);
-            ck(e);
-            ck(cudaEventCreateWithFlags(&plan->done, cudaEventDisableTiming));
-            plan->launches = launches;
-            plan->give_back();
-            c.plan = std::move(plan);
+                // Capture every group's work into one graph, each group on its own
+                // branch: the groups' persistent launches run back to back on the
+                // GPU, the next group's blocks filling the SMs that the previous
+                // group's tail frees. (One kernel over all layer counts was built
+                // and measured twice: with every solver inlined, its single
+                // register allocation spilled 0.6-1.6 KB of stack per thread; with
+                // each count's solver out of line, it ran 4.45 against 6.52 Mpx/s
+                // on a 64-image batch, its one shared-memory size set by the
+                // largest layer count holding every group's occupancy down.)
+                if (!c.fork) {
+                    ck(cudaEventCreateWithFlags(&c.fork, cudaEventDisableTiming));
+                    for (int q = 0; q < kMaxLayers; ++q) {
+                        ck(cudaStreamCreateWithFlags(&c.branch[q], cudaStreamNonBlocking));
+                        ck(cudaEventCreateWithFlags(&c.join[q], cudaEventDisableTiming));
+                    }
+                }
+                cudaGraph_t graph = nullptr;
+                ck(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
+                int launches = 0;
+                try {
+                    ck(cudaEventRecord(c.fork, s));
+                    for (size_t gi = 0; gi < gs.size(); ++gi) {
+                        auto& G = gs[gi];
+                        cudaStream_t s = c.branch[gi];   // this group's branch (shadows the call's stream)
+                        ck(cudaStreamWaitEvent(s, c.fork, 0));
+                        ck(cudaMemsetAsync(G.queues, 0, 8 * sizeof(uint32_t), s));
+                        if (G.order) {
+                            // The group's queue grouped by colour (order.cu).
+                            ck(launch_group_order(G.fp.jobs, G.fp.job_count, int(G.total), G.order_cells, G.order, c.sms,
+                                                  s));
+                            launches += 4;
+                        }
+                        for (auto& [k, w] : G.infer) {
+                            ck(launch_mlp_infer(G.net, jobs[k].image, jobs[k].width, jobs[k].height, G.L, w, G.counts + 3,
+                                                c.sms, s));
+                            ++launches;
+                        }
+                        if (so.precision == UNBLENDING_PRECISION_FP64) {
+                            ck(launch_solve_batch_fp64(G.L, G.v64, ctl, G.fp, 128, c.sms, s));
+                            ++launches;
+                            if (!G.infer.empty()) {
+                                ck(launch_solve_batch_fp64(G.L, G.v64, ctl, G.re, 128, c.sms, s));
+                                ++launches;
+                            }
+                        } else {
+                            ck(launch_solve_batch_fp32(G.L, G.variant, ctl32, G.fp, G.threads, c.sms, s));
+                            ++launches;
+                            if (so.resolve_misses && !G.infer.empty()) {
+                                ck(launch_solve_batch_fp32(G.L, G.variant, ctl32, G.mid, G.threads, c.sms, s));
+                                ++launches;
+                            }
+                            if (so.resolve_misses) {
+                                ck(launch_solve_batch_fp64(G.L, G.v64, ctl_re, G.re, 128, c.sms, s));
+                                ++launches;
+                            } else {
+                                ck(cudaMemcpyAsync(G.counts + 1, G.counts, sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
+                            }
+                        }
+                        ck(cudaEventRecord(c.join[gi], s));
+                    }
+                    for (size_t gi = 0; gi < gs.size(); ++gi) ck(cudaStreamWaitEvent(s, c.join[gi], 0));
+                } catch (...) {
+                    cudaStreamEndCapture(s, &graph);
+                    if (graph) cudaGraphDestroy(graph);
+                    throw;
+                }
+                ck(cudaStreamEndCapture(s, &graph));
+                cudaError_t e = cudaGraphInstantiate(&plan.exec, graph, 0);
+                cudaGraphDestroy(graph);
+                ck(e);
+                ck(cudaEventCreateWithFlags(&plan.done, cudaEventDisableTiming));
+                plan.launches = launches;
+            });
         }
         BatchPlan& P = *c.plan;
         ck(cudaEventRecord(c.ev[0], s));
