@@ -44,18 +44,6 @@
 
 namespace unb {
 
-// RN(1/b) from the hardware's approximation, without the branch to a slow path
-// that __drcp_rn takes, so that it overlaps the code around it (with
-// __drcp_rn the two passes of the 1024x1024 five-layer image took 1.03 times as
-// long).
-__device__ __forceinline__ double reciprocal(double b) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    y = refine_reciprocal(b, y);
-    const bool ones = (uint32_t(__double2hiint(b)) | 0xfff00000u) == 0xffffffffu && __double2loint(b) == -1;
-    return __hiloint2double(__double2hiint(y), ones ? 1 : __double2loint(y));
-}
-
 // Blend values of three channels of one layer (blend_value of each).
 __device__ __forceinline__ void blend_value3(int mode, const double* s, const double* d, double* f) {
     const double eps = 1e-5;

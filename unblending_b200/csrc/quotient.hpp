@@ -1,6 +1,7 @@
 // Correctly rounded division by a shared reciprocal.
 #pragma once
 #include <cmath>
+#include <cstdint>
 
 #ifdef __CUDACC__
 #define UNB_HOST_DEVICE __host__ __device__ __forceinline__
@@ -41,5 +42,19 @@ UNB_HOST_DEVICE double refine_reciprocal(double b, double y) {
     y = fma(y, fma(-b, y, 1.0), y);
     return fma(y, fma(-b, y, 1.0), y);
 }
+
+#ifdef __CUDACC__
+// RN(1/b) from the hardware's approximation, without the branch to a slow path
+// that __drcp_rn takes, so that it overlaps the code around it (with
+// __drcp_rn the two passes of the 1024x1024 five-layer image took 1.03 times as
+// long).
+__device__ __forceinline__ double reciprocal(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = refine_reciprocal(b, y);
+    const bool ones = (uint32_t(__double2hiint(b)) | 0xfff00000u) == 0xffffffffu && __double2loint(b) == -1;
+    return __hiloint2double(__double2hiint(y), ones ? 1 : __double2loint(y));
+}
+#endif
 
 }  // namespace unb
