@@ -419,15 +419,22 @@ template <class T, int L, bool REFINE, bool BATCH> struct LaneSolver {
         for (int c = 0; c < 4; ++c) t[c] = REFINE && c == 3 ? x[c] : clamp01(madd<T>(s, d[c], x[c]));
     }
 
+    // Layer l of the best point, at x or at the trial point of step best_step, to
+    // its record (x as it is: a step of zero along an infinite d would not be x).
+    __device__ __forceinline__ void store_best(int l, const T* x, const T* d) const {
+        const bool at_x = best_at == kBestAtX;
+        T t[4];
+        point(x, d, best_step, t);
+        store_rec(best_rec(l), at_x ? x[0] : t[0], at_x ? x[1] : t[1], at_x ? x[2] : t[2], at_x ? x[3] : t[3]);
+    }
+
     // Writes the best point to its records before x or d changes.
     __device__ __forceinline__ void save_best() {
-        const bool at_x = best_at == kBestAtX;
 #pragma unroll 1
         for (int l = 0; l < L; ++l) {
-            T x[4], d[4], t[4];
+            T x[4], d[4];
             get(kX, l, x); get(kD, l, d);
-            point(x, d, best_step, t);
-            store_rec(best_rec(l), at_x ? x[0] : t[0], at_x ? x[1] : t[1], at_x ? x[2] : t[2], at_x ? x[3] : t[3]);
+            store_best(l, x, d);
         }
         best_at = kBestStored;
     }
@@ -482,9 +489,7 @@ template <class T, int L, bool REFINE, bool BATCH> struct LaneSolver {
                     else if (!(as < tol_lo * w)) moved = moved || as > tol_hi * w || step_reaches(as, w, ctl.inner_tolerance);
                 }
                 if (best_lost) {
-                    T b[4];
-                    point(x, d, best_at == kBestAtX ? T(0.0) : best_step, b);
-                    store_rec(best_rec(l), b[0], b[1], b[2], b[3]);
+                    store_best(l, x, d);
                 }
                 store_rec(ring(next, 0, l), s[0], s[1], s[2], s[3]);
                 put(kX, l, t[0], t[1], t[2], t[3]);
