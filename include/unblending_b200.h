@@ -252,6 +252,7 @@ typedef struct unblending_image_job {
  * while the same job list is submitted again. The kernel variant and block
  * size of each group come from a timing sweep on a pixel sample, cached per
  * layer count. Results equal those of unblending_unmix_device per image.
+ * At most 2^31 - 1 pixels per layer count (more: UNBLENDING_INVALID_ARGUMENT).
  * Synchronous when stats is non-NULL. */
 UNBLENDING_API int32_t unblending_unmix_batch_device(
     const unblending_image_job* jobs, int32_t count, const unblending_options* options,

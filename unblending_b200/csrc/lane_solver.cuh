@@ -1164,7 +1164,8 @@ template <class T, int L, bool REFINE, bool BATCH> struct LaneSolver {
                     write = what == kFinished;
                 }
                 // Finished pixels are written, and the lanes without a pixel
-                // take the next queue entries together.
+                // take the next queue entries together. (The queue's head passes
+                // the total, which may be close to 2^31, by up to one a lane.)
                 for (;;) {
                     if (write) { store(o, skipped, capped); write = false; capped = false; state = kLaneFetch; }
                     const unsigned want = __ballot_sync(full, state == kLaneFetch);
@@ -1175,7 +1176,7 @@ template <class T, int L, bool REFINE, bool BATCH> struct LaneSolver {
                     base = __shfl_sync(full, base, leader);
                     if (state == kLaneFetch) {
                         const int job = base + __popc(want & ((1u << lane) - 1u));
-                        if (job >= total) state = kLaneIdle;
+                        if (uint32_t(job) >= uint32_t(total)) state = kLaneIdle;
                         else {
                             state = kLaneEnd;
                             what = kNextStart;

@@ -66,9 +66,9 @@ __device__ __forceinline__ uint32_t colour_cell(const double* rgb, int bits) {
 }
 
 __global__ void order_count(const OrderSource src, int count, int bits, uint32_t* __restrict__ cells) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < uint32_t(count); k += gridDim.x * blockDim.x) {
         int32_t value;
-        atomicAdd(&cells[colour_cell(src.rgb(k, value), bits)], 1u);
+        atomicAdd(&cells[colour_cell(src.rgb(int(k), value), bits)], 1u);
     }
 }
 
@@ -138,9 +138,9 @@ __global__ void __launch_bounds__(kScanThreads) order_chunk_scan(uint32_t* __res
 
 __global__ void order_scatter(const OrderSource src, int count, int bits, uint32_t* __restrict__ cells,
                               int32_t* __restrict__ order) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < uint32_t(count); k += gridDim.x * blockDim.x) {
         int32_t value;
-        const double* rgb = src.rgb(k, value);
+        const double* rgb = src.rgb(int(k), value);
         order[atomicAdd(&cells[colour_cell(rgb, bits)], 1u)] = value;
     }
 }

@@ -1319,12 +1319,13 @@ template <class T, int L, bool REFINE, int S, bool BATCH = false, int MODE = kPl
 
     // Pulls the next pixel: aBeginStart when it needs solving, aFetch again
     // after a pixel that is written without solving, aEval with `live`
-    // cleared when the queue is empty.
+    // cleared when the queue is empty. (The queue's head passes the total,
+    // which may be close to 2^31, by up to one a quad.)
     __device__ int fetch(int total, bool& live) {
         int job = 0;
         if (Q.q == 0) job = int(atomicAdd(a.queue, 1u));
         job = Q.from(job, 0);
-        if (job >= total) { phase = kIdle; live = false; return aEval; }
+        if (uint32_t(job) >= uint32_t(total)) { phase = kIdle; live = false; return aEval; }
         gidx = a.list ? a.list[job] : (a.order ? a.order[job] : a.first_pixel + job);
         int i = gidx;
         if constexpr (BATCH) {

@@ -1093,6 +1093,11 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
         }
         groups[J.layer_count].push_back(k);
     }
+    for (auto& [L, members] : groups) {
+        int64_t total = 0;
+        for (int k : members) total += int64_t(specs[k].pixels);
+        if (total > std::numeric_limits<int>::max()) return UNBLENDING_INVALID_ARGUMENT;   // (32-bit queue indices)
+    }
     // Plan key: everything the captured graph depends on.
     std::vector<unsigned char> key;
     auto put = [&](const void* p, size_t bytes) {
