@@ -145,6 +145,7 @@ struct SolveArgs {
     // each job's layer models come from `models` (Models<T> entries).
     const BatchJob* jobs = nullptr;
     int job_count = 0;
+    int groups = 1;   // groups of the batch: launches that share the GPU with this one
     const void* models = nullptr;
     // Optional totals over the launch: evaluations with a value, with a gradient.
     unsigned long long* tally = nullptr;

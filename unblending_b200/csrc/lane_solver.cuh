@@ -1130,9 +1130,23 @@ template <class T, int L, bool REFINE, bool BATCH> struct LaneSolver {
         const int total = a.list ? min(*a.list_count, a.list_limit) : (a.pixel_count >= 0 ? a.pixel_count : a.n);
         // A small launch spreads its pixels over all blocks, and in a block over
         // its warps: the fewer pixels share a block's phases, the shorter the
-        // last one's chain.
+        // last one's chain. Not so the groups of a batch, which run side by side
+        // (also as re-solves, of a few thousand hard pixels each): spread over all
+        // blocks, each would hold the others off the SMs until its last chain
+        // ends. A group whose pixels fit its share of the blocks leaves the
+        // rest of them to the others, unless it has less than two pixels a block
+        // there. FP32 batches, ms, every block / share / quad re-solve: 162,387
+        // pixels in four groups (16,086 misses) 17.4 / 13.6 / 16.0, 26,674
+        // (3,700) 8.6 / 6.3 / 7.8, 3,241 (830) 4.5 / 4.9 / 6.9; FP64 batches, every
+        // block / share: 26,674 8.1 / 4.9, 3,941 5.6 / 4.1, 2,029 3.6 / 4.1.
         static_assert(kLaneBlock == 128, "four warps a block");
-        if (int64_t((threadIdx.x & 31u) << 2 | threadIdx.x >> 5) * gridDim.x >= total) state = kLaneIdle;
+        int blocks = gridDim.x;
+        if constexpr (BATCH) {
+            const int share = max(1, blocks / a.groups);
+            if (total > 2 * share && total <= share * kLaneBlock) blocks = share;
+            if (int(blockIdx.x) >= blocks) return;
+        }
+        if (int64_t((threadIdx.x & 31u) << 2 | threadIdx.x >> 5) * blocks >= total) state = kLaneIdle;
         // Lanes waiting for each phase, one byte a phase (trial, direction,
         // gradient, outer step), counted over the block with one barrier, in
         // two buffers in turn.

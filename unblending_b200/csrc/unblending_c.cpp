@@ -1217,6 +1217,7 @@ int32_t unblending_unmix_batch_device(const unblending_image_job* jobs, int32_t 
                     SolveArgs& a = G.fp;
                     a.n = int(total);
                     a.jobs = d_table; a.job_count = int(table.size());
+                    a.groups = int(groups.size());
                     a.opaque = specs[members[0]].opaque; a.smooth = 0;
                     a.queue = G.queues;
                     a.miss_list = lists; a.miss_count = G.counts + 0;
