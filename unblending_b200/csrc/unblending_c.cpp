@@ -1667,12 +1667,18 @@ int32_t unblending_unmix_device_noalloc(int32_t width, int32_t height, const dou
         // eight layers, 9.7 / 49 / 116 -> 7.1 / 29 / 48 ms against the quad kernel
         // with its history in shared memory. That kernel (same results) serves
         // quad variants, which would need an array of their own, and re-solves
-        // whose lists leave too little room.
+        // whose lists leave too little room. Where the two are equal depends on
+        // the layers (the fewer, the more quads an SM holds); quads / lanes where
+        // many pixels miss, by blocks: two layers 49: 0.82, 65: 0.97, 75: 1.06;
+        // three 49: 0.91, 59: 1.04, 75: 1.21; four 37: 0.83, 50: 1.03, 60: 1.17;
+        // five 37: 0.89, 44: 0.98, 50: 1.01-1.14; six 37: 0.96, 44: 1.10; seven
+        // and eight 37: 1.23-1.28. So the line is at 74, 65, 57, 49, 41 blocks for
+        // two to six layers, and 37 from there.
         const bool fp64 = so.precision == UNBLENDING_PRECISION_FP64;
         const size_t lists = fp64 ? 0 : (2 * n * sizeof(int32_t) + 255) / 256 * 256;
         const int lane_block_count = int(std::min<size_t>(size_t(lane_blocks(L, sms, false)),
                                                           (bytes - 256 - lists) / lane_block_bytes(L, false)));
-        const bool lanes = lane_solve(so) && lane_block_count >= sms / 4;
+        const bool lanes = lane_solve(so) && lane_block_count >= std::max(sms / 4, sms * (11 - L) / 18);
         const int v64 = lanes ? kFp64Lanes : variant_global_history(true, fp64_variant(so, false)) ? 0 : fp64_variant(so, false);
         auto attach_fp64 = [&](SolveArgs& x) {
             if (!lanes) return;
