@@ -33,7 +33,9 @@ enum {
  * (unblending.cpp:351-353). */
 typedef struct unblending_solver_options {
     uint32_t struct_size;
-    int32_t precision;          /* UNBLENDING_PRECISION_*, default FP64 */
+    int32_t precision;          /* UNBLENDING_PRECISION_*, default FP64. FP32 is the faster for single images
+                                   (1.1x at 1024x1024, five layers) and the slower for batches, whose FP32 solves
+                                   run on the quad kernels (64 images: 14.8 against 24.7 Mpx/s) */
     int32_t starts;             /* 1..3 solver starts, default 1 */
     int32_t radius;             /* refinement radius; < 0 selects 60 * min(w, h) / 1000 */
     double epsilon;             /* guided-filter regularizer, default 1e-4 */
@@ -41,8 +43,10 @@ typedef struct unblending_solver_options {
     int32_t inner, outer;       /* iteration caps, default 256 and 22 */
     double inner_tolerance;     /* default 5e-3 */
     double outer_tolerance;     /* feasibility tolerance on |C|, default 5e-3 */
-    int32_t threads_per_block;  /* 0 selects the tuned default */
-    int32_t kernel_variant;     /* FP32 solve: -1 default, one pixel per lane (batches: a tuned quad variant);
+    int32_t threads_per_block;  /* 0 (default): one pixel per lane, 128 threads. 32, 64, 96 or 128: the quad
+                                   kernels with blocks of that size (same results, up to four times slower) */
+    int32_t kernel_variant;     /* FP32 solve: -1 default, one pixel per lane (batches: a tuned quad variant;
+                                   the allocation-free pass: 3);
                                    quad variants: 0 history in registers; 1/2 history in shared
                                    memory with registers capped for 4/5 blocks per SM; 3 as 1 with the evaluation
                                    rolled over the layers; 4 history in global memory, rolled, 5 blocks per SM;
@@ -251,7 +255,7 @@ typedef struct unblending_image_job {
  * inference and FP64 re-solves) are captured into one CUDA graph, replayed
  * while the same job list is submitted again. The kernel variant and block
  * size of each group come from a timing sweep on a pixel sample, cached per
- * layer count. Results equal those of unblending_unmix_device per image.
+ * layer count (FP32 precision). Results equal those of unblending_unmix_device per image.
  * At most 2^31 - 1 pixels per layer count (more: UNBLENDING_INVALID_ARGUMENT).
  * Synchronous when stats is non-NULL. */
 UNBLENDING_API int32_t unblending_unmix_batch_device(

@@ -91,7 +91,9 @@ __host__ __device__ constexpr int lane_smem_bytes(int L, bool fp32) {
 // take 18.7 (640x480, first pass); four layers and fewer spill at four blocks
 // (38 against 24 ms on 680x834). FP32, 1024x1024 five layers, first pass +
 // refinement in ms by blocks per SM: three 23.1 + 16.4, four 20.0 + 13.9, five
-// 21.3 + 15.5, six 26.4 + 16.6 (spills).
+// 21.3 + 15.5, six 26.4 + 16.6 (spills); 800x600, solves of nine outer steps,
+// three / four: six layers 18.1 + 15.9 / 16.3 + 13.7, seven 23.6 + 22.9 /
+// 24.2 + 23.5, eight 23.8 + 21.7 / 23.8 + 21.8.
 __host__ __device__ constexpr int lane_blocks_per_sm(int L, bool fp32) { return fp32 ? (L <= 6 ? 4 : 3) : L <= 5 ? 3 : 2; }
 __host__ __device__ constexpr int lane_blocks(int L, int sms, bool fp32) { return lane_blocks_per_sm(L, fp32) * sms; }
 __host__ __device__ constexpr size_t lane_block_bytes(int L, bool fp32) {

@@ -4,7 +4,10 @@
 // (FP64: rounded multiplies and adds; FP32: its fused and approximate forms; a
 // pixel's sums over the three channels and the alphas are added in the tree in
 // which a quad's lanes add theirs), so outputs, statuses and counters equal
-// its kernels' bit for bit in both precisions. Figures below are FP64's.
+// its kernels' bit for bit in both precisions. (Two edges are not the same
+// operations: a zero numerator's quotient loses its sign, and FP64 steps of
+// 2^-537.5 to 2^-537 count as no motion. Neither reaches an output that any
+// test has seen.) Figures below are FP64's.
 //
 // Why one pixel per lane: on a quad, all four lanes repeat the composite alpha
 // chain and the 3x3 colour prior, lane 3 idles through the colour arithmetic,
@@ -22,16 +25,18 @@
 // trial, and the other actions run when a share of the block's lanes waits
 // for them (or none has a trial). With each warp on its own schedule, the
 // instruction cache thrashed between the phases' code (85-100 KB; 4 to 7 cycles
-// of fetch stall per issue, 75 + 45 ms for the two passes of the 1024x1024
-// five-layer image); with the block in phase the stall is 0.3 cycles (34 + 22
-// ms, against 134 + 99 on quads). Even a block whose warps meet once a trip
-// only is slower (measured at 42 + 26 ms: 47 + 28).
+// of fetch stall per issue): putting the block in phase took the two passes of
+// the 1024x1024 five-layer image from 75 + 45 to 53 + 33 ms. (The quads take
+// 130 + 88 ms; the steps since the phases, 35 + 21. The fetch stall is now 0.46
+// and 0.34 cycles per issue.) Even a block whose warps meet once a trip only is
+// slower (measured at 42 + 26 ms: 47 + 28).
 //
-// What bounds it (1024x1024, five layers, first pass): latency at three warps
-// per scheduler (the shared memory and registers that a pixel's state and the
-// direction's loops take) and lanes that wait for a phase: 43 % of issue slots,
-// 38 % of the FP64 pipe, 13.5 of 32 lanes active. Trials take 42 % of the time,
-// directions 30 %, gradients 13 %, the meetings 15 %, outer steps 3 %.
+// What bounds it (a 512x512 image of five layers, first pass and refinement):
+// latency at three warps per scheduler (the shared memory and registers that a
+// pixel's state and the direction's loops take) and lanes that wait for a
+// phase: 49 and 51 % of issue slots, 45 % of the FP64 pipe, 14 to 15 of 32
+// lanes active. At 1024x1024 trials take 38 and 52 % of the time, directions 34
+// and 14 %, gradients 13 %, outer steps 4 and 6 %, the meetings 10 and 15 %.
 //
 // An accepted trial needs its gradient once; the lane's values repeat their
 // evaluation during the next trial phase, beside the lanes that evaluate
@@ -518,8 +523,10 @@ template <class T, int L, bool REFINE, bool BATCH> struct LaneSolver {
         }
         const T norm = sum(nn), value = energy + sum(terms), slope = sum(sl);
 
-        // A trial that does not move (whose sum of squared motions is zero:
-        // squares below the smallest number) ends the attempt, unevaluated.
+        // A trial that does not move (whose sum of squared motions is zero)
+        // ends the attempt, unevaluated. FP32: squares that round to zero, up to
+        // 2^-75; FP64 by the high word, below 2^-537 (squares round to zero
+        // below 2^-537.5).
         if (!at_x && largest < (kFast ? 0x1a000001u : 0x1e600000u)) { attempt_failed(); return; }
         const T tol2 = ctl.outer_tolerance * ctl.outer_tolerance;
         const bool feasible = norm < tol2;

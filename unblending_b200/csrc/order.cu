@@ -1,15 +1,16 @@
 // Work-queue order of a solve launch: the pixels grouped by colour.
 //
-// A quad's path through the method (which actions it takes, how many
-// line-search trials, how many outer steps) depends on the pixel's target
-// colour; in the first pass it is a function of that colour alone. The
-// lockstep kernel runs every action that any quad of a warp needs, with the
-// other quads waiting, so a warp whose eight pixels have similar colours
-// wastes fewer trips. The queue therefore hands out pixels in a Morton
-// (Z-curve) order of their RGB quantized to `bits` bits a channel (4 to 7,
-// about one cell per pixel for the launch's pixel count):
-// consecutive queue indices, which the quads of a warp pull at about the same
-// time, are pixels of nearby colours. Each pixel's solve reads only its own
+// A pixel's path through the method (which actions it takes, how many
+// line-search trials, how many outer steps) depends on its target colour; in
+// the first pass it is a function of that colour alone. A lane kernel's block
+// runs one action at a time for the lanes that are at it, and a quad kernel's
+// warp every action that any of its quads needs, with the others waiting, so
+// pixels of similar colours side by side waste less. The queue therefore hands
+// out pixels in a Morton (Z-curve) order of their RGB quantized to `bits` bits
+// a channel (4 to 7, about one cell per pixel for the launch's pixel count):
+// consecutive queue indices, which a warp pulls at about the same time, are
+// pixels of nearby colours (1024x1024, five layers, lanes, first pass: 51.1 ms
+// in image order, 48.2 in colour order). Each pixel's solve reads only its own
 // inputs, so the order changes the speed and never the results.
 //
 // A counting sort over the 2^(3*bits) colour cells: count, exclusive scan

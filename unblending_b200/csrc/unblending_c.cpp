@@ -422,7 +422,7 @@ int32_t resolve_solver(const unblending_solver_options* in, unblending_solver_op
     return UNBLENDING_OK;
 }
 
-// FP32 kernel variant measured on B200 (FP32 solve of the first pass /
+// FP32 kernel variant on quads, measured on B200 (FP32 solve of the first pass /
 // refinement, ms; 1024x1024, 5 layers | 6 layers with colour noise): history
 // in shared memory, registers capped for 4 blocks per SM 56.6 / 62.7 |
 // 133 / 116; capped for 5 blocks 54.1 / 73.6 | 158 / 181; capped for 4 blocks
@@ -431,7 +431,7 @@ int32_t resolve_solver(const unblending_solver_options* in, unblending_solver_op
 // 48.8 -> 44.6 ms.
 int default_fp32_variant(int L, bool refine) { (void)L; return refine ? 5 : 3; }
 
-// FP64 kernel variant measured on B200 (1024x1024, 5 layers; re-solve of the
+// FP64 kernel variant on quads, measured on B200 (1024x1024, 5 layers; re-solve of the
 // FP32 misses, first pass / refinement, ms): shared history uncapped 91 / 130;
 // global history with x, g, d and the evaluation's per-layer intermediates in
 // shared memory (evaluation rolled over the layers), capped for 3 blocks:
@@ -457,11 +457,11 @@ int fp64_variant(const unblending_solver_options& so, bool refine) {
 // on quads: unless the caller names a quad variant or a block size. Lanes are
 // the faster at every size, by the length of the last pixels' serial chains in
 // the smallest launches (a launch spreads its pixels over all warps) and by
-// throughput in the large ones. Lanes / quads, ms, first pass and refinement:
-// three layers, 64 pixels 0.6 / 0.8 and 0.3 / 0.7, 5,184 1.7 / 2.1 and 1.5 / 3.0,
-// 65,536 2.0 / 4.1 and 2.0 / 4.6; five layers, 576 2.7 / 4.6 and 2.0 / 6.5,
-// 1,048,576 34 / 134 and 22 / 99; eight layers, 576 3.6 / 9.2 and 3.0 / 9.2, 65,536
-// 11 / 57 and 8.7 / 28.
+// throughput in the large ones. Lanes / quads (variants 3 and 7), ms, first
+// pass and refinement: the three-layer configuration, 64 pixels 0.36 / 0.88 and
+// 0.42 / 1.26, 5,184 1.27 / 2.05 and 1.17 / 3.05, 65,536 2.0 / 4.7 and 1.8 / 4.9; the
+// five-layer one, 576 1.7 / 3.4 and 1.7 / 5.0, 1,048,576 34.9 / 130 and 21.4 / 88; eight
+// layers, 576 3.2 / 9.5 and 3.0 / 11.4, 65,536 8.1 / 44 and 6.9 / 18.5.
 bool lane_solve(const unblending_solver_options& so) { return so.fp64_variant < 0 && so.threads_per_block == 0; }
 
 // Bytes of a global-memory L-BFGS history array for L layers and values of
